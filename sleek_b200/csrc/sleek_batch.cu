@@ -161,7 +161,7 @@ int sleek_batch_plan_create(const sleek_batch_item* items, int n, int decompress
     g.njobs = m;
     g.chunks = total;
     g.ws_bytes = p->decompress ? static_cast<size_t>(8 * (HDR_WORDS + total + 2 * m))
-                               : static_cast<size_t>(8 * (HDR_WORDS + total));
+                               : static_cast<size_t>(8 * (HDR_WORDS + total + m));
     if (cudaMalloc(&g.d_jobs, sizeof(sleek::BatchJob) * m) != cudaSuccess ||
         cudaMalloc(&g.d_cb, sizeof(long long) * (m + 1)) != cudaSuccess ||
         cudaMemcpy(g.d_jobs, jobs.data(), sizeof(sleek::BatchJob) * m, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -229,7 +229,7 @@ int sleek_batch_plan_set_items(sleek_batch_plan* plan, const sleek_batch_item* i
   g.njobs = n;
   g.chunks = total;
   g.ws_bytes = plan->decompress ? static_cast<size_t>(8 * (HDR_WORDS + total + 2 * n))
-                                : static_cast<size_t>(8 * (HDR_WORDS + total));
+                                : static_cast<size_t>(8 * (HDR_WORDS + total + n));
   plan->ws_bytes = g.ws_bytes;
   return SLEEK_OK;
 }
@@ -273,6 +273,7 @@ int sleek_batch_plan_run(sleek_batch_plan* plan, void* d_workspace, size_t works
       a.chunk_base = g.d_cb;
       a.njobs = g.njobs;
       a.ws = ws;
+      a.starts = ws + HDR_WORDS + g.chunks;
       e = sleek::launch_encode_batch(a, grid_for(plan, g.chunks), st);
     }
     if (e != cudaSuccess) {

@@ -2,7 +2,7 @@
 //
 // Host-side argument checks, grid sizing from the occupancy of the kernels on
 // the current device, workspace handling and error-bound derivation.  All
-// compute happens in sleek_kernels.cu; there is no CPU fallback.
+// compute happens in sleek_encode.cu and sleek_kernels.cu; there is no CPU fallback.
 #include <cstdint>
 #include <cstring>
 #include <map>
@@ -29,7 +29,7 @@ constexpr int BUCKETS = 64;  // input sizes by their base-2 logarithm
 
 // what the single-buffer calls of one kind launch for one size bucket
 struct Choice {
-  int shape = 0;  // launch shape (sleek_kernels.cu: EncShape*, DecShape*)
+  int shape = 0;  // launch shape (EncShape*, DecShape*)
   int ctas = 0;   // CTAs per SM, 0 = as many as fit
 };
 

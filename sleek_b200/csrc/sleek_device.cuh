@@ -135,6 +135,36 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, uint32_t
       : "memory");
 }
 
+// 1-D bulk copy shared -> global (16-byte aligned addresses and size), in the
+// calling thread's current bulk group.
+__device__ __forceinline__ void tma_store_1d(void* dst, const void* src, uint32_t bytes)
+{
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes)
+               : "memory");
+}
+
+// brings `bytes` (a multiple of 16, at a 16-byte aligned address) into L2
+__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes)
+{
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// the thread's bulk stores have read their shared memory
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// the thread's bulk stores are complete
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// Asynchronous copy of N = 4, 8 or 16 bytes global -> shared, of which the first
+// `have` are read and the rest zero-filled.
+template <int N>
+__device__ __forceinline__ void cp_async(void* dst, const void* src, int have)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_u32(dst)), "l"(src), "n"(N), "r"(have)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __device__ __forceinline__ void fence_proxy_async_smem()
 {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -255,31 +285,33 @@ struct WsPhase {
 // ----------------------------------------------------------------------------
 // The reference's forward step, on the rotated word v with exponent field
 // E = v >> 24: if E != 0, subtract 2^31, then subtract one more exponent unit if
-// the field became 0 or the top bit is set.  Case by case that adds 0 (E = 0),
-// 2^31 - 2^24 (1 <= E <= 0x80) or 2^31 (E > 0x80) mod 2^32, which is how it is
-// computed here (equal on all 2^32 inputs).
-__device__ __forceinline__ uint32_t fwd(uint32_t v)
+// the field became 0 or the top bit is set; then (v << 1) ^ (v >> 31 arithmetic).
+// Case by case the sum adds 0 (E = 0), 2^31 - 2^24 (1 <= E <= 0x80) or 2^31
+// (E > 0x80) mod 2^32, and only the middle case ends with the top bit set.  With
+// t = 2 v mod 2^32 that is t, or ~(t - 2^25) in the middle case, which is where
+// v - 2^24 is non-negative as a signed number (equal on all 2^32 inputs).
+__device__ __forceinline__ uint32_t fwd(uint32_t x)
 {
-  v = (v << 1) | (v >> 31);
-  v += v < 0x01000000u ? 0u : (v < 0x81000000u ? 0x7f000000u : 0x80000000u);
-  return (v << 1) ^ static_cast<uint32_t>(static_cast<int32_t>(v) >> 31);
+  const uint32_t v = __funnelshift_l(x, x, 1);
+  const uint32_t t = v + v;
+  return static_cast<int32_t>(v - 0x01000000u) >= 0 ? 0x01ffffffu - t : t;
 }
 
-// 64-bit lossless forward transform on 32-bit halves: the exponent test and
-// both subtractions touch only the high word (no borrow crosses into the low
-// word), the rotate and the final shift are funnel shifts.
-__device__ __forceinline__ uint64_t fwd(uint64_t v)
+// The same step on 64-bit values (11-bit exponent field), on 32-bit halves: the
+// case and the subtraction touch only the high word, so the low word of t is
+// inverted or kept.
+__device__ __forceinline__ uint64_t fwd(uint64_t x)
 {
-  const uint32_t h = static_cast<uint32_t>(v >> 32);
-  const uint32_t l = static_cast<uint32_t>(v);
-  uint32_t nh = __funnelshift_l(l, h, 1);        // rotate left by 1
-  const uint32_t nl = __funnelshift_l(h, l, 1);
-  // the same step on the 11-bit field: adds 0, 2^31 - 2^21 or 2^31
-  nh += nh < 0x00200000u ? 0u : (nh < 0x80200000u ? 0x7fe00000u : 0x80000000u);
-  const uint32_t sg = static_cast<uint32_t>(static_cast<int32_t>(nh) >> 31);
-  const uint32_t oh = __funnelshift_l(nl, nh, 1) ^ sg;  // (v << 1) ^ (v >> 63 arithmetic)
-  const uint32_t ol = (nl << 1) ^ sg;
-  return (static_cast<uint64_t>(oh) << 32) | ol;
+  const uint32_t h = static_cast<uint32_t>(x >> 32);
+  const uint32_t l = static_cast<uint32_t>(x);
+  const uint32_t nl = __funnelshift_l(h, l, 1);  // low word of v: rotated left by 1
+  uint32_t th = __funnelshift_l(l, h, 2);        // high word of t (v's shifted left once more)
+  uint32_t tl = nl + nl;
+  if (static_cast<int32_t>(h + h - 0x00200000u) >= 0) {  // v's lowest high bit does not matter here
+    th = 0x003fffffu - th;
+    tl = ~tl;
+  }
+  return (static_cast<uint64_t>(th) << 32) | tl;
 }
 
 __device__ __forceinline__ uint32_t inv(uint32_t v)
@@ -609,6 +641,174 @@ __device__ __forceinline__ long long lookback(const uint64_t* flags, long long i
 }
 
 // ----------------------------------------------------------------------------
+// Encode's placement of chunks.  A chunk publishes its size in a 32-bit flag (0 = not
+// yet) and adds it to the sum of its group of 64 consecutive chunks (count in the
+// high half).  One warp per CTA, the scanner, follows the groups in order, up to 32
+// per poll (2,048 chunks, about as many as are ever in flight), and keeps the
+// prefix before each in a ring in shared memory; a chunk's own warp adds the flags
+// of its group before it (one 8-byte load per lane).  So a chunk is placed about one
+// round trip to L2 after its predecessors are sized, however many they are, and 148
+// warps poll the group sums.
+// ----------------------------------------------------------------------------
+constexpr int GROUP = 64;  // chunks per group
+constexpr int RING = 128;  // groups whose prefixes a CTA keeps
+
+// words (8 bytes) of the flags and group sums of `chunks` chunks: at most `chunks`
+// (the sums are not used where there is only one group)
+__host__ __device__ constexpr long long scan_words(long long chunks)
+{
+  return (chunks + 1) / 2 + (chunks > GROUP ? (chunks + GROUP - 1) / GROUP : 0);
+}
+
+struct ScanRing {
+  uint64_t base[RING];  // sizes of all chunks before group i, at i % RING
+  long long known;      // groups whose prefix is known: 0 .. known
+  int gone;             // warps that have left their chunk loop
+};
+
+struct ChunkScan {
+  uint32_t* flags;  // per chunk
+  uint64_t* sums;   // per group: sum of sizes | count << 32
+  long long chunks;
+  volatile ScanRing* ring;
+
+  __device__ ChunkScan(uint64_t* region, long long chunks_, ScanRing* ring_)
+      : flags(reinterpret_cast<uint32_t*>(region)), sums(region + (chunks_ + 1) / 2), chunks(chunks_), ring(ring_)
+  {
+  }
+
+  // one thread: the size of chunk `idx` is known
+  __device__ void publish(long long idx, uint32_t csize) const
+  {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(flags + idx), "r"(csize) : "memory");
+    if (chunks > GROUP)
+      asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(sums + idx / GROUP), "l"((1ull << 32) | csize)
+                   : "memory");
+  }
+
+  // this lane's share of the sizes of chunks [b, e) of one group, and whether they are published
+  __device__ bool part(long long b, long long e, int lane, uint32_t* sum) const
+  {
+    const long long i = b / GROUP * GROUP + 2 * lane;
+    const bool in0 = i >= b && i < e, in1 = i + 1 >= b && i + 1 < e;
+    uint64_t f = 0;
+    if (in0 || in1) f = ld_relaxed_u64(reinterpret_cast<const uint64_t*>(flags + i));
+    const uint32_t f0 = in0 ? static_cast<uint32_t>(f) : 0u;
+    const uint32_t f1 = in1 ? static_cast<uint32_t>(f >> 32) : 0u;
+    *sum = f0 + f1;
+    return (!in0 || f0) && (!in1 || f1);
+  }
+
+  // The scanner warp: until the prefix of the last group is known or `warps` warps
+  // have left (their own waits are bounded).
+  __device__ void follow(int warps) const
+  {
+    const int lane = threadIdx.x & 31;
+    const long long last = (chunks + GROUP - 1) / GROUP - 1;
+    long long f = 0;
+    uint64_t before = 0;
+    while (f < last && ring->gone < warps) {
+      const long long h = f + lane;
+      const uint64_t v = h < last ? ld_relaxed_u64(sums + h) : 0ull;
+      const unsigned no = __ballot_sync(0xffffffffu, (v >> 32) != GROUP);
+      const int n = no ? __ffs(no) - 1 : 32;
+      if (n == 0) continue;
+      uint32_t incl = static_cast<uint32_t>(v);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += x;
+      }
+      if (lane < n) ring->base[(h + 1) % RING] = before + incl;
+      before += __shfl_sync(0xffffffffu, incl, n - 1);
+      f += n;
+      __threadfence_block();
+      __syncwarp();
+      if (lane == 0) ring->known = f;
+    }
+  }
+
+  // The prefix before chunk `idx`, modulo 8 or 16, if every chunk after the last
+  // group known so far is compressed (size 2 modulo that); a hint only.
+  __device__ long long guess(long long idx) const
+  {
+    const long long own = idx / GROUP;
+    long long g = ring->known;
+    g = g < own ? g : own;
+    return (g > 0 ? static_cast<long long>(ring->base[g % RING]) : 0ll) + 2 * (idx - g * GROUP);
+  }
+
+  // One warp: the sum of the sizes of all chunks before `idx`, or -1 when a wait
+  // exceeded the limit or another CTA reported an error in the counter block.
+  // Where `from` lies in the own group, only of chunks [from, idx).
+  __device__ long long prefix(long long idx, long long from, const uint64_t* hdr) const
+  {
+    const int lane = threadIdx.x & 31;
+    const long long own = idx / GROUP;
+    long long b = own * GROUP;
+    bool need_base = own > 0;
+    if (from >= b) {
+      b = from;
+      need_base = false;
+    }
+    bool need_own = idx > b;
+    long long excl = 0;
+    unsigned long long t0 = 0;
+    int polls = 0;
+    while (true) {
+      if (need_own) {
+        uint32_t s;
+        const bool ok = part(b, idx, lane, &s);
+        if (__all_sync(0xffffffffu, ok)) {
+          excl += __reduce_add_sync(0xffffffffu, s);
+          need_own = false;
+        }
+      }
+      if (need_base && ring->known >= own) {
+        __threadfence_block();
+        uint64_t v = ring->base[own % RING];
+        __threadfence_block();
+        if (ring->known + 32 >= own + RING) {  // the entry may be gone: add up the groups
+          uint64_t s = 0;
+          for (long long h = lane; h < own; h += 32) s += ld_relaxed_u64(sums + h) & 0xffffffffull;
+          v = static_cast<uint64_t>(warp_sum(static_cast<long long>(s)));
+        }
+        excl += static_cast<long long>(v);
+        need_base = false;
+      }
+      if (!need_own && !need_base) return excl;
+      // a predecessor has not published yet: back off, bounded in time
+      if (++polls == 256) {
+        t0 = globaltimer_ns();
+      } else if (polls > 256 && (polls & 255) == 0) {
+        const bool late = globaltimer_ns() - t0 > SPIN_TIMEOUT_NS;
+        const bool failed = ld_relaxed_u64(&hdr[WS_STATUS]) != 0ull;
+        if (__any_sync(0xffffffffu, late || failed)) return -1;
+      }
+      __nanosleep(64);
+    }
+  }
+
+  // One warp: the value another warp puts at `p` (never 0), or 0 when the wait gave up.
+  __device__ static uint64_t await(const uint64_t* p, const uint64_t* hdr)
+  {
+    unsigned long long t0 = 0;
+    for (int polls = 0;; ++polls) {
+      const uint64_t v = ld_relaxed_u64(p);
+      if (__all_sync(0xffffffffu, v != 0ull)) return __shfl_sync(0xffffffffu, v, 0);
+      if (polls == 256) {
+        t0 = globaltimer_ns();
+      } else if (polls > 256 && (polls & 255) == 0) {
+        const bool late = globaltimer_ns() - t0 > SPIN_TIMEOUT_NS;
+        const bool failed = ld_relaxed_u64(&hdr[WS_STATUS]) != 0ull;
+        if (__any_sync(0xffffffffu, late || failed)) return 0ull;
+      }
+      __nanosleep(64);
+    }
+  }
+};
+
+// ----------------------------------------------------------------------------
 // Shifted store: writes `len` bytes from 16-byte aligned shared memory `src`
 // to the arbitrary global byte address `dst`.  Whole aligned 16-byte granules
 // get one vector store each, funnel-shifted from two aligned shared loads; the
@@ -716,6 +916,23 @@ __device__ __forceinline__ uint64_t extract_bits64(const uint32_t* w, int pos, i
   const uint32_t hi = __funnelshift_r(w1, w2, sh);
   const uint64_t v = (static_cast<uint64_t>(hi) << 32) | lo;
   return ln >= 64 ? v : (v & ((1ull << ln) - 1ull));
+}
+
+// ----------------------------------------------------------------------------
+// host
+// ----------------------------------------------------------------------------
+// Sets the dynamic shared memory limit of `k` once per device.
+template <typename K>
+static cudaError_t ensure_smem_attr(K k, int bytes, unsigned long long* done_mask)
+{
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (__atomic_load_n(done_mask, __ATOMIC_ACQUIRE) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) __atomic_fetch_or(done_mask, bit, __ATOMIC_RELEASE);
+  return e;
 }
 
 }  // namespace sleek

@@ -1,0 +1,799 @@
+// sleek_encode.cu -- sm_100a encode kernel (one buffer, and batches of buffers).
+//
+// Replaces d_encode (include/sleek_common_gpu.h:474-559, 989-1074 of the reference).
+// One warp takes a chunk from its first byte to its last, alone: it takes a ticket
+// (atomic), has the 16 KB chunk copied to its stage of shared memory (one TMA bulk
+// copy), turns the values into codes in place and ORs them into the subchunks' bit
+// widths, publishes the chunk's size, packs the codes in place, waits for its place
+// in the stream, and stores the packed chunk with one bulk copy.  Fourteen such warps
+// share an SM, each with its own stage, with no barrier between them: while some wait
+// for memory, others compute, so neither a CTA-wide barrier per chunk nor a pipeline
+// of producer, compute and store warps is needed.  A fifteenth warp, the scanner,
+// follows the sizes of all chunks (ChunkScan, sleek_device.cuh).
+//
+// What bounds it: instruction issue and the 14 stages an SM has room for.  A chunk
+// costs 2,800 warp instructions (f64 lossless; 5,250 when eight warps shared a chunk,
+// because each of them waited at barriers, scanned the widths and shifted the packed
+// bytes to their place), and its stage is taken for 8-10 us.  Every wait between the
+// published size and the store counts against the stages, so the pack comes before
+// the wait for the place, at the alignment the place is expected to have.
+// (302 MB f64 field: lossless 144 -> 114 us, eb 1e-4 129 -> 90 us; 26 MB f32 field,
+// eb 1e-3: 24.1 -> 16.7 us; 67 MB f32 signal, lossless: 44.6 -> 34.8 us.)
+#include <type_traits>
+
+#include "sleek_device.cuh"
+#include "sleek_launch.h"
+
+namespace sleek {
+
+// KIND: bit 0 = 64-bit values, bit 1 = lossy
+template <int KIND>
+using EncVal = typename std::conditional<(KIND & 1) != 0, uint64_t, uint32_t>::type;
+
+constexpr int EW_IN = 64;               // the chunk's bytes begin here in a warp's stage
+constexpr int EW_STAGE = EW_IN + CS;    // room before them for the packed chunk's widths and alignment
+
+// ---- phase A: values to codes in place, and the subchunks' widths ------------------
+
+constexpr int EW_G = 4;  // subchunks whose loads, maps and reductions overlap
+
+// Quantizes one group's values (EW_G subchunks, this lane's 16 bytes of each) when
+// all of the warp's are ordinary: |v| small enough that the code needs at most 30
+// bits (f64) or is not an escape (f32).  False (nothing written) otherwise.
+__device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], uint32_t (&o)[EW_G], float limit, float inv_scale)
+{
+  bool odd = false;
+#pragma unroll
+  for (int u = 0; u < EW_G; ++u) {
+    odd |= !(fabsf(__uint_as_float(w[u].x)) < limit);
+    odd |= !(fabsf(__uint_as_float(w[u].y)) < limit);
+    odd |= !(fabsf(__uint_as_float(w[u].z)) < limit);
+    odd |= !(fabsf(__uint_as_float(w[u].w)) < limit);
+  }
+  if (__any_sync(0xffffffffu, odd)) return false;
+  auto one = [&](uint32_t v) {
+    const uint32_t e = __float2uint_rz(__fmaf_rd(fabsf(__uint_as_float(v)), inv_scale, 0.5f));
+    return static_cast<uint32_t>(max(static_cast<int>(2u * e - (v >> 31)), 0));
+  };
+#pragma unroll
+  for (int u = 0; u < EW_G; ++u) {
+    w[u].x = one(w[u].x);
+    w[u].y = one(w[u].y);
+    w[u].z = one(w[u].z);
+    w[u].w = one(w[u].w);
+    o[u] = w[u].x | w[u].y | w[u].z | w[u].w;
+  }
+  return true;
+}
+
+__device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], uint32_t (&o)[EW_G], float limit, double inv_scale)
+{
+  bool odd = false;
+#pragma unroll
+  for (int u = 0; u < EW_G; ++u) {
+    // the high words, ordered like floats (those that are no number as a float are large)
+    odd |= !(fabsf(__uint_as_float(w[u].y)) < limit);
+    odd |= !(fabsf(__uint_as_float(w[u].w)) < limit);
+  }
+  if (__any_sync(0xffffffffu, odd)) return false;
+  auto one = [&](uint32_t l, uint32_t h) {
+    const double v = fabs(__hiloint2double(static_cast<int>(h), static_cast<int>(l)));
+    const uint32_t e = __double2uint_rz(__fma_rd(v, inv_scale, 0.5));
+    return static_cast<uint32_t>(max(static_cast<int>(2u * e - (h >> 31)), 0));
+  };
+#pragma unroll
+  for (int u = 0; u < EW_G; ++u) {
+    w[u].x = one(w[u].x, w[u].y);
+    w[u].z = one(w[u].z, w[u].w);
+    w[u].y = 0u;
+    w[u].w = 0u;
+    o[u] = w[u].x | w[u].z;
+  }
+  return true;
+}
+
+// One warp: the staged chunk's values become codes in place (each lane reads and
+// writes its own 16 bytes of every subchunk); returns the bit width of subchunk
+// `lane`.
+template <int KIND>
+__device__ __forceinline__ int encode_values(uint8_t* data, const QParams& q, int lane)
+{
+  using T = EncVal<KIND>;
+  constexpr bool LOSSY = (KIND & 2) != 0;
+  uint32_t hi_or = 0, lo_or = 0;  // OR of the codes of subchunk `lane`
+  // ordinary values of the quantizer (see quant_group)
+  float limit = 0.0f;
+  typename std::conditional<sizeof(T) == 4, float, double>::type inv_scale = 0;
+  if constexpr (LOSSY) {
+    if constexpr (sizeof(T) == 4) {
+      limit = q.eb_e ? __uint_as_float(static_cast<uint32_t>(q.thr_e) << 23) : 0.0f;
+      inv_scale = __uint_as_float(static_cast<uint32_t>(277 - q.thr_e) << 23);
+    } else {
+      limit = q.eb_e ? __uint_as_float(static_cast<uint32_t>(q.thr_e - 23) << 20) : 0.0f;
+      inv_scale = __longlong_as_double(static_cast<long long>(2098 - q.thr_e) << 52);
+    }
+  }
+#pragma unroll 1
+  for (int i0 = 0; i0 < SC; i0 += EW_G) {
+    uint4 w[EW_G];
+    uint32_t o[EW_G], oh[EW_G];
+    uint4* const p = reinterpret_cast<uint4*>(data + i0 * 512 + lane * 16);
+#pragma unroll
+    for (int u = 0; u < EW_G; ++u) w[u] = p[32 * u];
+    bool done = false;
+    if constexpr (LOSSY) done = quant_group(w, o, limit, inv_scale);
+    if (done) {
+#pragma unroll
+      for (int u = 0; u < EW_G; ++u) oh[u] = 0u;
+    } else {
+#pragma unroll
+      for (int u = 0; u < EW_G; ++u) {
+        if constexpr (sizeof(T) == 4) {
+          w[u].x = encode_value<LOSSY>(w[u].x, q);
+          w[u].y = encode_value<LOSSY>(w[u].y, q);
+          w[u].z = encode_value<LOSSY>(w[u].z, q);
+          w[u].w = encode_value<LOSSY>(w[u].w, q);
+          o[u] = w[u].x | w[u].y | w[u].z | w[u].w;
+          oh[u] = 0u;
+        } else {
+          const uint64_t a = encode_value<LOSSY>((static_cast<uint64_t>(w[u].y) << 32) | w[u].x, q);
+          const uint64_t b = encode_value<LOSSY>((static_cast<uint64_t>(w[u].w) << 32) | w[u].z, q);
+          w[u] = make_uint4(static_cast<uint32_t>(a), static_cast<uint32_t>(a >> 32), static_cast<uint32_t>(b),
+                            static_cast<uint32_t>(b >> 32));
+          o[u] = w[u].x | w[u].z;
+          oh[u] = w[u].y | w[u].w;
+        }
+      }
+      if constexpr (sizeof(T) == 8) {
+#pragma unroll
+        for (int u = 0; u < EW_G; ++u) {
+          const uint32_t r = __reduce_or_sync(0xffffffffu, oh[u]);
+          if (lane == i0 + u) hi_or = r;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < EW_G; ++u) {
+      p[32 * u] = w[u];
+      const uint32_t r = __reduce_or_sync(0xffffffffu, o[u]);
+      if (lane == i0 + u) lo_or = r;
+    }
+  }
+  return hi_or ? 64 - __clz(hi_or) : 32 - __clz(lo_or);
+}
+
+// ---- phase B: codes to the packed chunk, in place ----------------------------------
+
+// Packs the chunk one subchunk after the other.  `at` is the word being filled
+// next; `carry` (lane 0) holds the bits already set in that word: the packed bits
+// begin in the middle of a word when the chunk's place in the stream does.
+struct Packer {
+  uint32_t* at;
+  uint32_t carry;
+  int half;  // bits of the first word that precede the packed bits (0 or 16)
+  int lane;
+
+  // The lane's run of R bits (32 <= R <= 128, low bits first in x0..x3) goes to bit
+  // lane * R of the subchunk.  Every word holds bits of at most two lanes: a lane
+  // stores the words that its run completes and hands the rest to the next one.
+  template <int MINR, int MAXR>
+  __device__ __forceinline__ void put(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3, int R)
+  {
+    const int rs = half + lane * R;
+    const int s = rs & 31;
+    const int t = s + R;
+    const uint32_t y0 = x0 << s;
+    const uint32_t y1 = __funnelshift_l(x0, x1, s);
+    const uint32_t y2 = __funnelshift_l(x1, x2, s);
+    uint32_t y3 = 0u, tail;
+    if constexpr (MAXR > 64) {
+      y3 = __funnelshift_l(x2, x3, s);
+      const uint32_t y4 = __funnelshift_l(x3, 0u, s);
+      tail = t < 96 ? y2 : (t < 128 ? y3 : y4);
+      if (MINR < 64 && t < 64) tail = y1;
+    } else {
+      tail = t < 64 ? y1 : y2;
+    }
+    const uint32_t r = __shfl_sync(0xffffffffu, tail, (lane + 31) & 31);
+    uint32_t* const d = at + (rs >> 5);
+    d[0] = y0 | (lane == 0 ? carry : r);
+    if (MINR >= 64 || t >= 64) d[1] = y1;
+    if (MAXR > 64) {
+      if (t >= 96) d[2] = y2;
+      if (t >= 128) d[3] = y3;
+    }
+    carry = r;
+    at += R;
+  }
+
+  // Runs of R < 32 bits: adjacent lanes' runs are joined until they have 32 bits
+  // or more, then every 2nd, 4th, ... lane stores.
+  __device__ __forceinline__ void put_short(uint32_t run, int R)
+  {
+    int w = R, step = 1;
+    while (2 * w < 32) {
+      run |= __shfl_down_sync(0xffffffffu, run, step) << w;
+      w *= 2;
+      step *= 2;
+    }
+    const uint32_t n = __shfl_down_sync(0xffffffffu, run, step);
+    const uint32_t x0 = run | (n << w);
+    const uint32_t x1 = __funnelshift_l(n, 0u, w);
+    w *= 2;
+    step *= 2;
+    const int rs = half + lane * R;
+    const int s = rs & 31;
+    const int t = s + w;
+    const uint32_t y0 = x0 << s;
+    const uint32_t y1 = __funnelshift_l(x0, x1, s);
+    const uint32_t y2 = __funnelshift_l(x1, 0u, s);
+    const uint32_t r = __shfl_sync(0xffffffffu, t < 64 ? y1 : y2, (lane - step) & 31);
+    if ((lane & (step - 1)) == 0) {
+      uint32_t* const d = at + (rs >> 5);
+      d[0] = y0 | (lane == 0 ? carry : r);
+      if (t >= 64) d[1] = y1;
+    }
+    carry = r;
+    at += R;
+  }
+
+  // A run of R bits (16 <= R < 64) per lane, without a branch on R: runs shorter than
+  // a word are joined in pairs, and then every other lane stores.
+  __device__ __forceinline__ void put_any(uint32_t x0, uint32_t x1, int R)
+  {
+    const bool pair = R < 32;
+    const uint32_t n = __shfl_down_sync(0xffffffffu, x0, 1);
+    if (pair) {
+      x0 |= n << R;
+      x1 = __funnelshift_l(n, 0u, R);
+    }
+    const int w = pair ? 2 * R : R;
+    const int step = pair ? 2 : 1;
+    const int rs = half + lane * R;
+    const int s = rs & 31;
+    const int t = s + w;
+    const uint32_t y0 = x0 << s;
+    const uint32_t y1 = __funnelshift_l(x0, x1, s);
+    const uint32_t y2 = __funnelshift_l(x1, 0u, s);
+    const uint32_t r = __shfl_sync(0xffffffffu, t < 64 ? y1 : y2, (lane - step) & 31);
+    uint32_t* const d = at + (rs >> 5);
+    if ((lane & (step - 1)) == 0) {
+      d[0] = y0 | (lane == 0 ? carry : r);
+      if (t >= 64) d[1] = y1;
+    }
+    carry = r;
+    at += R;
+  }
+
+  // one subchunk of 32-bit codes, this lane's four
+  __device__ __forceinline__ void put32(const uint4 w, int ln)
+  {
+    if (ln == 0) return;
+    if (ln == 32) {
+      put<64, 128>(w.x, w.y, w.z, w.w, 128);
+    } else if (ln >= 16) {
+      wide32(w, ln);
+    } else {
+      const uint32_t m = 1u << ln;
+      const uint32_t a = w.y * m + w.x, b = w.w * m + w.z;  // at most 30 bits each
+      if (ln >= 8) put<32, 64>(b * (m * m) + a, __funnelshift_l(b, 0u, 2 * ln), 0u, 0u, 4 * ln);
+      else put_short(b * (m * m) + a, 4 * ln);
+    }
+  }
+  // 4 <= ln <= 15
+  __device__ __forceinline__ void narrow32(const uint4 w, int ln)
+  {
+    const uint32_t m = 1u << ln;
+    const uint32_t a = w.y * m + w.x, b = w.w * m + w.z;
+    put_any(b * (m * m) + a, __funnelshift_l(b, 0u, 2 * ln), 4 * ln);
+  }
+  // 16 <= ln <= 31
+  __device__ __forceinline__ void wide32(const uint4 w, int ln)
+  {
+    const uint32_t m = 1u << ln;
+    const uint32_t a0 = w.y * m + w.x, a1 = __funnelshift_l(w.y, 0u, ln);
+    const uint32_t b0 = w.w * m + w.z, b1 = __funnelshift_l(w.w, 0u, ln);
+    const int k = 2 * ln - 32;
+    put<64, 128>(a0, b0 * (1u << k) + a1, __funnelshift_l(b0, b1, k), __funnelshift_l(b1, 0u, k), 4 * ln);
+  }
+
+  // one subchunk of 64-bit codes, this lane's two
+  __device__ __forceinline__ void put64(const uint4 w, int ln)
+  {
+    if (ln == 0) return;
+    if (ln == 64) put<64, 128>(w.x, w.y, w.z, w.w, 128);
+    else if (ln >= 32) wide64(w, ln);
+    else if (ln >= 16) narrow64(w, ln);
+    else put_short(w.z * (1u << ln) + w.x, 2 * ln);
+  }
+  // 32 <= ln <= 63
+  __device__ __forceinline__ void wide64(const uint4 w, int ln)
+  {
+    const int k = ln - 32;
+    put<64, 128>(w.x, w.z * (1u << k) + w.y, __funnelshift_l(w.z, w.w, k), __funnelshift_l(w.w, 0u, k), 2 * ln);
+  }
+  // 16 <= ln <= 31
+  __device__ __forceinline__ void narrow64(const uint4 w, int ln)
+  {
+    put<32, 64>(w.z * (1u << ln) + w.x, __funnelshift_l(w.z, 0u, ln), 0u, 0u, 2 * ln);
+  }
+  // 8 <= ln <= 31
+  __device__ __forceinline__ void any64(const uint4 w, int ln)
+  {
+    put_any(w.z * (1u << ln) + w.x, __funnelshift_l(w.z, 0u, ln), 2 * ln);
+  }
+};
+
+// One warp: packs the codes staged at `stg + EW_IN` into the chunk's bytes at
+// `stg + a` (a < 16, even: the chunk's place in the stream modulo 16): the 32 width
+// bytes, the packed bits, the int16 trailer.  In place, subchunk by subchunk: the
+// packed bytes of a subchunk end before the codes of the next one begin, and a
+// lane's stores follow an exchange that every lane enters with its codes loaded.
+template <typename T>
+__device__ __forceinline__ void pack_chunk(uint8_t* stg, int a, int ln, int osize, int lane)
+{
+  constexpr int B = static_cast<int>(sizeof(T));
+  stg[a + lane] = static_cast<uint8_t>(ln);
+  Packer k;
+  k.lane = lane;
+  k.half = (a & 2) * 8;
+  k.at = reinterpret_cast<uint32_t*>(stg + ((a + 32) & ~3));
+  // the last two widths share the first word with the packed bits
+  const uint32_t l2 = __shfl_sync(0xffffffffu, ln, 30) | (__shfl_sync(0xffffffffu, ln, 31) << 8);
+  k.carry = k.half ? l2 : 0u;
+  const unsigned wide = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 16 && ln < 32) : (ln >= 32 && ln < 64));
+  const unsigned narrow = B == 8 ? __ballot_sync(0xffffffffu, ln >= 16 && ln < 32) : 0u;
+  const unsigned any = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 4 && ln < 16) : (ln >= 8 && ln < 32));
+#pragma unroll 1
+  for (int i0 = 0; i0 < SC; i0 += EW_G) {
+    uint4 w[EW_G];
+    int l[EW_G];
+#pragma unroll
+    for (int u = 0; u < EW_G; ++u) {
+      w[u] = *reinterpret_cast<const uint4*>(stg + EW_IN + (i0 + u) * 512 + lane * 16);
+      l[u] = __shfl_sync(0xffffffffu, ln, i0 + u);
+    }
+    constexpr unsigned ALL = (1u << EW_G) - 1u;
+    if (((wide >> i0) & ALL) == ALL) {
+#pragma unroll
+      for (int u = 0; u < EW_G; ++u) {
+        if constexpr (B == 4) k.wide32(w[u], l[u]);
+        else k.wide64(w[u], l[u]);
+      }
+    } else if (B == 8 && ((narrow >> i0) & ALL) == ALL) {
+#pragma unroll
+      for (int u = 0; u < EW_G; ++u) k.narrow64(w[u], l[u]);
+    } else if (((any >> i0) & ALL) == ALL) {
+#pragma unroll
+      for (int u = 0; u < EW_G; ++u) {
+        if constexpr (B == 4) k.narrow32(w[u], l[u]);
+        else k.any64(w[u], l[u]);
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < EW_G; ++u) {
+        if constexpr (B == 4) k.put32(w[u], l[u]);
+        else k.put64(w[u], l[u]);
+      }
+    }
+  }
+  if (lane == 0) {
+    if (k.half) *k.at = (k.carry & 0xffffu) | (static_cast<uint32_t>(osize) << 16);
+    else *reinterpret_cast<int16_t*>(k.at) = static_cast<int16_t>(osize);
+  }
+}
+
+// Stores the packed chunk at `src` (byte `a` of its 16-byte granule) to its place: one
+// bulk copy of the whole granules where the place has the same alignment, else 16-byte
+// stores put together from the staged words; the two granules shared with the
+// neighbouring chunks two bytes at a time (sizes and places are even).
+__device__ __forceinline__ void store_chunk(uint8_t* dst, const uint8_t* src, int a, int csize, int lane)
+{
+  const int al = static_cast<int>(reinterpret_cast<uintptr_t>(dst) & 15u);
+  const int b = (16 - al) & 15;             // chunk bytes before the first whole granule
+  const int e = ((al + csize) & ~15) - al;  // and up to the end of the last
+  if (al == a) {
+    if (lane == 0) {
+      tma_store_1d(dst + b, src + b, static_cast<uint32_t>(e - b));
+      bulk_commit();
+    }
+  } else if (((al ^ a) & 7) == 0) {
+#pragma unroll 4
+    for (int o = b + 16 * lane; o < e; o += 512) {
+      const uint2 x = *reinterpret_cast<const uint2*>(src + o), y = *reinterpret_cast<const uint2*>(src + o + 8);
+      *reinterpret_cast<uint4*>(dst + o) = make_uint4(x.x, x.y, y.x, y.y);
+    }
+  } else {
+    const int sh = ((a + b) & 2) * 8;
+#pragma unroll 2
+    for (int o = b + 16 * lane; o < e; o += 512) {
+      const uint32_t* const p = reinterpret_cast<const uint32_t*>(src + o - (sh >> 3));
+      const uint32_t w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = p[4];
+      *reinterpret_cast<uint4*>(dst + o) = make_uint4(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh),
+                                                      __funnelshift_r(w2, w3, sh), __funnelshift_r(w3, w4, sh));
+    }
+  }
+  const int o = lane < 16 ? 2 * lane : e + 2 * (lane - 16);
+  if (lane < 16 ? o < b : o < csize)
+    *reinterpret_cast<uint16_t*>(dst + o) = *reinterpret_cast<const uint16_t*>(src + o);
+}
+
+// ---- the kernel --------------------------------------------------------------------
+
+// What a warp needs to know about its chunk.
+struct EncChunk {
+  const uint8_t* in;  // its first byte
+  uint8_t* out;       // the buffer's stream
+  long long* outsize;
+  long long g;        // chunk id across the launch
+  long long c;        // chunk index within its buffer
+  long long chunks;   // chunks of the buffer
+  long long insize;   // bytes of the buffer
+  QParams q;
+  int kind;
+  int osize;
+};
+
+// Copies the chunk's bytes to `dst` (zero-padded to a full chunk) and waits for
+// them: one TMA bulk copy, or, where the input is not 16-byte aligned or the chunk
+// is partial, asynchronous copies of the widest elements the address allows.
+__device__ __forceinline__ bool load_chunk(uint8_t* dst, const uint8_t* in, int osize, uint64_t* bar, uint32_t& par,
+                                           int lane)
+{
+  const unsigned mis = static_cast<unsigned>(reinterpret_cast<uintptr_t>(in)) & 15u;
+  if (mis == 0u && osize == CS) {
+    if (lane == 0) {
+      mbar_arrive_expect_tx(bar, CS);
+      tma_load_1d(dst, in, CS, bar);
+    }
+    const bool ok = mbar_wait_bounded(bar, par);
+    par ^= 1u;
+    return !__any_sync(0xffffffffu, !ok);
+  }
+  auto copy = [&](auto width) {
+    constexpr int N = decltype(width)::value;
+#pragma unroll 8
+    for (int k = 0; k < CS / (32 * N); ++k) {
+      const int o = (k * 32 + lane) * N;
+      const int have = min(max(osize - o, 0), N);
+      cp_async<N>(dst + o, have ? in + o : in, have);
+    }
+  };
+  if (mis == 0u) copy(std::integral_constant<int, 16>{});
+  else if (mis == 8u) copy(std::integral_constant<int, 8>{});
+  else copy(std::integral_constant<int, 4>{});
+  cp_async_wait_all();
+  __syncwarp();
+  return true;
+}
+
+template <int KIND, bool BATCH, int NW, int MINB>
+__global__ void __launch_bounds__((NW + 1) * 32, MINB)
+    k_encode(const typename std::conditional<BATCH, BatchEncArgs, EncArgs>::type a)
+{
+  extern __shared__ __align__(128) uint8_t smem[];
+  uint64_t* const bars = reinterpret_cast<uint64_t*>(smem + NW * EW_STAGE);
+  long long* const cb = reinterpret_cast<long long*>(bars + NW);
+  const int tid = threadIdx.x;
+  const int lane = tid & 31;
+  const int warp = tid >> 5;
+  uint8_t* const stg = smem + warp * EW_STAGE;
+  uint64_t* const bar = bars + warp;
+
+  const WsPhase ph = [&]() {
+    if constexpr (BATCH) return WsPhase::fixed(a.ws);
+    else return WsPhase::of(a.ws, a.flag_cap);
+  }();
+  uint64_t* const hdr = ph.hdr;
+  if constexpr (BATCH) {
+    for (int i = tid; i <= a.njobs; i += (NW + 1) * 32) cb[i] = a.chunk_base[i];
+  }
+  __shared__ unsigned long long s_first;
+  __shared__ ScanRing ring;
+  // The first tickets are taken for the whole CTA, as many as an even share of a
+  // small input leaves it; a ticket is only ever held by a running warp.
+  unsigned long long* const tick = reinterpret_cast<unsigned long long*>(&a.ws[WS_TICKET]);
+  const long long total = [&]() -> long long {
+    if constexpr (BATCH) return a.chunk_base[a.njobs];
+    else return (a.insize + CS - 1) / CS;
+  }();
+  const long long share = (total + gridDim.x - 1) / gridDim.x;
+  const int first_n = static_cast<int>(share < NW ? share : NW);
+  if (tid == 0) {
+    s_first = atomicAdd(tick, static_cast<unsigned long long>(first_n));
+    for (int i = 0; i < NW; ++i) mbar_init(&bars[i], 1);
+    mbar_fence_init();
+    ring.known = 0;
+    ring.gone = 0;
+  }
+  __syncthreads();
+  const ChunkScan scan(ph.flags, total, &ring);
+
+  uint32_t par = 0;
+  auto next = [&]() -> long long {
+    unsigned long long t = 0;
+    if (lane == 0) t = atomicAdd(tick, 1ull);
+    return static_cast<long long>(__shfl_sync(0xffffffffu, t, 0));
+  };
+  if (warp == NW) {
+    scan.follow(NW);
+    if constexpr (!BATCH) ph.clear_other_share(lane);
+  } else {
+  long long t = warp < first_n ? static_cast<long long>(s_first) + warp : next();
+  while (t < total) {
+    EncChunk k;
+    long long seg = 0;
+    int job = 0;
+    if constexpr (BATCH) {
+      int lo = 0, hi = a.njobs - 1;  // last job whose first chunk id is <= t (empty jobs are skipped)
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (cb[mid] <= t) lo = mid;
+        else hi = mid - 1;
+      }
+      const BatchJob& j = a.jobs[lo];
+      seg = cb[lo];
+      job = lo;
+      k.g = t;
+      k.c = t - seg;
+      k.in = j.in + k.c * CS;
+      k.out = j.out;
+      k.outsize = j.outsize;
+      k.chunks = j.chunks;
+      k.insize = j.insize;
+      k.q = j.q;
+      k.kind = j.kind;
+    } else {
+      k.g = t;
+      k.c = t;
+      k.in = a.in + t * CS;
+      k.out = a.out;
+      k.outsize = a.outsize;
+      k.chunks = total;
+      k.insize = a.insize;
+      k.q = a.q;
+      k.kind = KIND;
+    }
+    k.osize = static_cast<int>(min(static_cast<long long>(CS), k.insize - k.c * CS));
+
+    if (!load_chunk(stg + EW_IN, k.in, k.osize, bar, par, lane)) {
+      if (lane == 0) set_status(hdr, ST_TIMEOUT, k.g);
+      break;
+    }
+    int ln;
+    if constexpr (KIND >= 0) {
+      ln = encode_values<KIND>(stg + EW_IN, k.q, lane);
+    } else {
+      switch (k.kind) {
+        case 0: ln = encode_values<0>(stg + EW_IN, k.q, lane); break;
+        case 1: ln = encode_values<1>(stg + EW_IN, k.q, lane); break;
+        case 2: ln = encode_values<2>(stg + EW_IN, k.q, lane); break;
+        default: ln = encode_values<3>(stg + EW_IN, k.q, lane); break;
+      }
+    }
+    const bool wide = (KIND >= 0 ? KIND : k.kind) & 1;
+    const int wtot = __reduce_add_sync(0xffffffffu, wide ? 2 * ln : 4 * ln);
+    const bool comp = 34 + 4 * wtot < k.osize;
+    const int csize = comp ? 34 + 4 * wtot : k.osize;
+    if (lane == 0) scan.publish(k.g, static_cast<uint32_t>(csize));
+    if (!comp) {  // stored as it came: fetched again (the codes took its place), mostly from L2
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (!load_chunk(stg + EW_IN, k.in, k.osize, bar, par, lane)) {
+        if (lane == 0) set_status(hdr, ST_TIMEOUT, k.g);
+        break;
+      }
+    }
+    // Packed before its place is known, at the alignment that it has if every chunk
+    // not placed yet is compressed (a compressed chunk's size is 2 mod 16 for 32-bit
+    // values, 2 mod 8 for 64-bit ones).
+    int al = 0;
+    if (comp) {
+      long long guess = 2 * k.c;
+      if constexpr (!BATCH) guess = scan.guess(k.g);
+      al = static_cast<int>((reinterpret_cast<uintptr_t>(k.out) + 8 + 2 * k.chunks + guess) & 15u);
+      if (wide) pack_chunk<uint64_t>(stg, al, ln, k.osize, lane);
+      else pack_chunk<uint32_t>(stg, al, ln, k.osize, lane);
+      fence_proxy_async_smem();
+      __syncwarp();
+    }
+    if constexpr (!BATCH) {
+      // The chunk about a full round of tickets ahead goes to L2, so that its warp's
+      // load takes one L2 round trip, not a queue at HBM that all later chunks' places
+      // would wait for.  After the pack, not before: at a kernel's start the first
+      // loads of all warps are still under way (302 MB f64 lossless: 108 us against 116
+      // with the prefetch right after the load and 110 without one).
+      const long long ahead = t + static_cast<long long>(gridDim.x) * NW;
+      if (lane == 0 && (ahead + 1) * CS <= a.insize && (reinterpret_cast<uintptr_t>(a.in) & 15u) == 0u)
+        prefetch_l2(a.in + ahead * CS, CS);
+    }
+    long long excl = scan.prefix(k.g, BATCH && k.c > 0 ? seg : 0, hdr);
+    if constexpr (BATCH) {
+      // the place within the buffer: relative to its first chunk, whose warp tells
+      // the others where it is unless they share its group
+      if (excl >= 0) {
+        uint64_t* const start = a.starts + job;
+        if (k.c == 0) {
+          if (lane == 0) st_relaxed_u64(start, FLAG_INC | static_cast<uint64_t>(excl));
+          excl = 0;
+        } else if (seg < k.g / GROUP * GROUP) {
+          const uint64_t v = ChunkScan::await(start, hdr);
+          excl = v ? excl - static_cast<long long>(v & FLAG_VAL) : -1;
+        }
+      }
+    }
+    if (excl < 0 || excl > k.c * CS) {
+      if (lane == 0) set_status(hdr, excl < 0 ? ST_TIMEOUT : ST_CAPACITY, k.g);
+      break;
+    }
+    if (lane == 0) {
+      if (k.c == k.chunks - 1) {
+        if constexpr (BATCH) {  // the buffer is complete: its header and size
+          *reinterpret_cast<long long*>(k.out) = k.insize;
+          *k.outsize = 8 + 2 * k.chunks + excl + csize;
+        } else {
+          hdr[WS_TOTAL] = static_cast<uint64_t>(excl + csize);
+        }
+      }
+      *reinterpret_cast<uint16_t*>(k.out + 8 + 2 * k.c) = static_cast<uint16_t>(csize);
+    }
+    uint8_t* const dst = k.out + 8 + 2 * k.chunks + excl;
+    if (comp) store_chunk(dst, stg + al, al, csize, lane);
+    else store_shifted<32>(dst, stg + EW_IN, csize, lane);
+    t = next();
+    // the stage is read before it is refilled
+    if (lane == 0) bulk_wait_read();
+    fence_proxy_async_smem();
+    __syncwarp();
+  }
+  if (lane == 0) {
+    atomicAdd(&ring.gone, 1);
+    bulk_wait();
+  }
+  }
+
+  // ---- epilogue: the last CTA out finishes the outputs -----------------------
+  __syncthreads();
+  __shared__ int last_cta;
+  if (tid == 0) {
+    __threadfence();
+    const unsigned long long d = atomicAdd(reinterpret_cast<unsigned long long*>(&a.ws[WS_DONE]), 1ull);
+    last_cta = d == gridDim.x - 1;
+    if (last_cta) __threadfence();
+  }
+  __syncthreads();
+  if (last_cta) {
+    const unsigned long long st = ld_relaxed_u64(&hdr[WS_STATUS]);
+    if constexpr (BATCH) {
+      // buffers without chunks get their header-only stream; an error anywhere
+      // turns every size into -status
+      for (int i = tid; i < a.njobs; i += (NW + 1) * 32) {
+        const BatchJob& j = a.jobs[i];
+        if (st) {
+          *j.outsize = -static_cast<long long>(st);
+        } else if (j.chunks == 0) {
+          *reinterpret_cast<long long*>(j.out) = 0;
+          *j.outsize = 8;
+        }
+      }
+    } else if (tid == 0) {
+      const long long tot = total ? static_cast<long long>(ld_relaxed_u64(&hdr[WS_TOTAL])) : 0ll;
+      *reinterpret_cast<long long*>(a.out) = a.insize;
+      *a.outsize = st ? -static_cast<long long>(st) : 8 + 2 * total + tot;
+      ph.finish(a.ws, scan_words(total));
+    }
+  }
+}
+
+// ---- launchers ---------------------------------------------------------------------
+
+// Launch shapes: warps (and stages) per CTA and CTAs per SM.  The largest CTA that
+// fits, one per SM, has the most chunks in flight and one scanner warp per SM; the
+// others leave room for kernels of other streams, or for the autotuner to pick.
+template <int NW_, int MINB_>
+struct EncShape {
+  static constexpr int NW = NW_;
+  static constexpr int MINB = MINB_;
+  static constexpr int NT = (NW + 1) * 32;  // + the scanner warp
+  static constexpr int SMEM = NW * EW_STAGE + 8 * NW;
+};
+using EncShape0 = EncShape<14, 1>;  // default
+using EncShape1 = EncShape<12, 1>;
+using EncShape2 = EncShape<6, 2>;
+using EncShape3 = EncShape<4, 3>;
+using EncShape4 = EncShape<8, 1>;
+constexpr int ENC_SHAPES = 5;
+using EncShapeBatch = EncShape<13, 1>;  // + the jobs' first chunk ids
+constexpr int ENC_BATCH_SMEM = EncShapeBatch::SMEM + 8 + 8 * (BATCH_MAX_JOBS + 1);
+
+template <int KIND, class S>
+static cudaError_t launch_enc_k(const EncArgs& a, int grid, cudaStream_t st)
+{
+  auto k = k_encode<KIND, false, S::NW, S::MINB>;
+  static unsigned long long attr = 0;
+  cudaError_t e = ensure_smem_attr(k, S::SMEM, &attr);
+  if (e != cudaSuccess) return e;
+  k<<<grid, S::NT, S::SMEM, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int KIND, class S>
+static int enc_occupancy()
+{
+  auto k = k_encode<KIND, false, S::NW, S::MINB>;
+  // the smem attribute must be set before the occupancy query counts dynamic smem
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+  int n = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, S::NT, S::SMEM);
+  return n;
+}
+
+template <int KIND>
+static cudaError_t launch_enc_kind(int shape, const EncArgs& a, int grid, cudaStream_t st)
+{
+  switch (shape) {
+    case 1: return launch_enc_k<KIND, EncShape1>(a, grid, st);
+    case 2: return launch_enc_k<KIND, EncShape2>(a, grid, st);
+    case 3: return launch_enc_k<KIND, EncShape3>(a, grid, st);
+    case 4: return launch_enc_k<KIND, EncShape4>(a, grid, st);
+    default: return launch_enc_k<KIND, EncShape0>(a, grid, st);
+  }
+}
+
+template <int KIND>
+static int enc_occupancy_kind(int shape)
+{
+  switch (shape) {
+    case 1: return enc_occupancy<KIND, EncShape1>();
+    case 2: return enc_occupancy<KIND, EncShape2>();
+    case 3: return enc_occupancy<KIND, EncShape3>();
+    case 4: return enc_occupancy<KIND, EncShape4>();
+    default: return enc_occupancy<KIND, EncShape0>();
+  }
+}
+
+cudaError_t launch_encode(int width, bool lossy, int shape, const EncArgs& a, int grid, cudaStream_t st)
+{
+  if (width == 4) return lossy ? launch_enc_kind<2>(shape, a, grid, st) : launch_enc_kind<0>(shape, a, grid, st);
+  return lossy ? launch_enc_kind<3>(shape, a, grid, st) : launch_enc_kind<1>(shape, a, grid, st);
+}
+
+int encode_blocks_per_sm(int width, bool lossy, int shape)
+{
+  if (width == 4) return lossy ? enc_occupancy_kind<2>(shape) : enc_occupancy_kind<0>(shape);
+  return lossy ? enc_occupancy_kind<3>(shape) : enc_occupancy_kind<1>(shape);
+}
+
+int encode_shape_count() { return ENC_SHAPES; }
+
+ShapeInfo encode_shape_info(int shape)
+{
+  switch (shape) {
+    case 1: return {EncShape1::NT, EncShape1::NW, EncShape1::NW, EncShape1::MINB};
+    case 2: return {EncShape2::NT, EncShape2::NW, EncShape2::NW, EncShape2::MINB};
+    case 3: return {EncShape3::NT, EncShape3::NW, EncShape3::NW, EncShape3::MINB};
+    case 4: return {EncShape4::NT, EncShape4::NW, EncShape4::NW, EncShape4::MINB};
+    default: return {EncShape0::NT, EncShape0::NW, EncShape0::NW, EncShape0::MINB};
+  }
+}
+
+cudaError_t launch_encode_batch(const BatchEncArgs& a, int grid, cudaStream_t st)
+{
+  auto k = k_encode<-1, true, EncShapeBatch::NW, EncShapeBatch::MINB>;
+  static unsigned long long attr = 0;
+  cudaError_t e = ensure_smem_attr(k, ENC_BATCH_SMEM, &attr);
+  if (e != cudaSuccess) return e;
+  k<<<grid, EncShapeBatch::NT, ENC_BATCH_SMEM, st>>>(a);
+  return cudaGetLastError();
+}
+
+int encode_batch_blocks_per_sm()
+{
+  auto k = k_encode<-1, true, EncShapeBatch::NW, EncShapeBatch::MINB>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ENC_BATCH_SMEM);
+  int n = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, EncShapeBatch::NT, ENC_BATCH_SMEM);
+  return n;
+}
+
+}  // namespace sleek

@@ -1,21 +1,5 @@
-// sleek_kernels.cu -- sm_100a encode / decode kernels (one buffer, and batches).
-//
-// Encode (replaces d_encode, include/sleek_common_gpu.h:474-559, 989-1074 of the
-// reference): persistent CTAs of 8 compute warps, a producer warp and a scanner
-// warp, 3 per SM.  The producer takes a chunk ticket (atomic, just in time) and
-// copies the 16 KB chunk into one of four shared-memory stages with a 1-D TMA bulk
-// copy, two chunks ahead.  Each compute warp loads 4 subchunks into registers,
-// transforms or quantizes them (value arithmetic restated from the reference) and
-// ORs them into bit widths; after the compute warps' one barrier per chunk every
-// warp derives the offsets it needs by warp reductions, thread 0 publishes the
-// chunk's size, and each warp packs its subchunks from registers into the stage
-// (funnel-shifted runs with one neighbour exchange; short runs by shared OR).  The
-// scanner looks back over the chunk flags as soon as the chunk has landed and
-// records its payload offset; the producer stores the packed chunk to the stream
-// (16-byte vector stores, consecutive lanes on consecutive granules) right before
-// it refills that stage, so the compute warps never wait for an offset.  A chunk
-// whose encoding is not smaller than its input is stored raw straight from the
-// staged copy (never re-read from HBM).
+// sleek_kernels.cu -- sm_100a decode kernels (one buffer, and batches); encode is in
+// sleek_encode.cu.
 //
 // Decode (replaces d_decode, :688-768, 1199-1279): CTAs take contiguous chunk
 // ranges in ticket order, sum their ranges' compressed sizes, look back over the
@@ -28,774 +12,6 @@
 #include "sleek_launch.h"
 
 namespace sleek {
-
-// Launch shape of the encode kernel: CW compute warps (each takes SC / CW
-// subchunks of a chunk) and ST shared-memory stages of one chunk each.  The
-// producer copies chunk k once the compute warps have sized chunk k - AHEAD, right
-// after storing the stage's previous chunk, k - ST (whose look-back thereby gets
-// ST - AHEAD chunks of compute time).  MINB is the CTAs per SM the registers are
-// budgeted for.  Every shape writes the same bytes.
-template <int CW_, int ST_, int MINB_>
-struct EncShape {
-  static constexpr int CW = CW_;
-  static constexpr int ST = ST_;
-  // the copy of chunk seq is issued once the compute warps have sized chunk seq - AHEAD
-  static constexpr int AHEAD = 2;
-  static constexpr int MINB = MINB_;
-  static constexpr int NT = (CW + 2) * 32;  // + a producer warp and a scanner warp
-  static constexpr int SPW = SC / CW;       // subchunks per compute warp
-  static_assert(SC % CW == 0 && AHEAD < ST, "shape");
-};
-// the shapes the library is built with (index = the C ABI's shape number)
-using EncShape0 = EncShape<8, 4, 3>;   // default: 10 warps, 66 KB, 3 CTAs per SM
-using EncShape1 = EncShape<16, 4, 2>;  // 18 warps, 66 KB, 2 CTAs per SM
-using EncShape2 = EncShape<4, 4, 3>;   // 6 warps, 66 KB, 3 CTAs per SM
-using EncShape3 = EncShape<8, 3, 3>;   // 10 warps, 3 stages (50 KB), 3 CTAs per SM
-using EncShape4 = EncShape<8, 5, 2>;   // 10 warps, 5 stages (83 KB), 2 CTAs per SM
-constexpr int ENC_SHAPES = 5;
-constexpr long long NO_CHUNK = 0x7fffffffffffffffll;
-
-// What the producer tells the compute and scanner warps about the chunk in a stage.
-struct EncMeta {
-  long long g;          // look-back flag index (chunk id across the launch), or NO_CHUNK
-  long long c;          // chunk index within its buffer
-  long long seg;        // flag index of the buffer's first chunk
-  long long chunks;     // chunks of the buffer
-  long long insize;     // bytes of the buffer
-  uint8_t* out;         // the buffer's stream
-  long long* outsize;   // the buffer's size output
-  long long excl;       // payload offset of the chunk (scanner), -1 after an error
-  QParams q;            // the buffer's quantizer parameters
-  int kind;             // bit 0: 64-bit values, bit 1: lossy
-  int osize;
-  int csize;
-  int comp;
-};
-
-template <int ST>
-struct EncMisc {
-  uint64_t full[ST];    // chunk bytes landed (TMA tx count)
-  uint64_t sized[ST];   // compressed size of the stage's chunk known (compute warps past phase A)
-  uint64_t placed[ST];  // payload offset of the stage's chunk known
-  uint64_t packed[ST];  // every compute warp has packed its share of the stage's chunk
-  EncMeta meta[ST];
-  int lnv[2][SC];  // subchunk bit widths, by chunk parity (a fast warp may write the next chunk's)
-};
-
-template <class S>
-constexpr int enc_smem()
-{
-  return S::ST * STAGE_BYTES + static_cast<int>((sizeof(EncMisc<S::ST>) + 127) / 128) * 128;
-}
-template <class S>
-constexpr int enc_batch_smem()
-{
-  return enc_smem<S>() + 8 * (BATCH_MAX_JOBS + 1);  // + the jobs' first chunk ids
-}
-
-// barrier among the CW compute warps only (named barrier 1), OR-reducing `pred`
-template <int CW>
-__device__ __forceinline__ bool cbar_or(bool pred)
-{
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.or.pred q, 1, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"(static_cast<uint32_t>(pred)), "n"(CW * 32)
-      : "memory");
-  return r != 0;
-}
-
-// ORs `v`, placed at bit offset `o` (< 96, warp-uniform) of a 128-bit run, into
-// the run's words x0..x3.
-__device__ __forceinline__ void place32(uint32_t v, int o, uint32_t& x0, uint32_t& x1, uint32_t& x2, uint32_t& x3)
-{
-  const int q = o >> 5;
-  const int r = o & 31;
-  const uint32_t lo = v << r;
-  const uint32_t hi = __funnelshift_l(v, 0u, r);  // bits that cross into the next word
-  if (q == 0) {
-    x0 |= lo;
-    x1 |= hi;
-  } else if (q == 1) {
-    x1 |= lo;
-    x2 |= hi;
-  } else {
-    x2 |= lo;
-    x3 |= hi;
-  }
-}
-
-// Packs one subchunk whose transformed values sit in registers: lane L holds
-// values P*L .. P*L+P-1 and writes the bit run [P*L*ln, P*(L+1)*ln) of the
-// subchunk's packed bits (LSB-first, 32-bit little-endian words at `pw`).
-template <typename T>
-__device__ __forceinline__ void pack_subchunk(uint32_t* pw, int ln, const T (&v)[16 / sizeof(T)], int lane)
-{
-  constexpr int P = 16 / static_cast<int>(sizeof(T));  // values per lane
-  constexpr int TB = 8 * static_cast<int>(sizeof(T));
-  if (ln == 0) return;
-  if (ln == TB) {  // verbatim: the lane's 16 bytes in place
-    uint32_t* d = pw + 4 * lane;
-    if constexpr (sizeof(T) == 4) {
-      if ((reinterpret_cast<uintptr_t>(d) & 15u) == 0u) {
-        *reinterpret_cast<uint4*>(d) = make_uint4(v[0], v[1], v[2], v[3]);
-      } else {
-        d[0] = v[0]; d[1] = v[1]; d[2] = v[2]; d[3] = v[3];
-      }
-    } else {
-      reinterpret_cast<uint2*>(d)[0] = make_uint2(static_cast<uint32_t>(v[0]), static_cast<uint32_t>(v[0] >> 32));
-      reinterpret_cast<uint2*>(d)[1] = make_uint2(static_cast<uint32_t>(v[1]), static_cast<uint32_t>(v[1] >> 32));
-    }
-    return;
-  }
-  const int R = P * ln;  // bits of the lane's run
-  const int rs = lane * R;
-  const int w0 = rs >> 5;
-  const int s = rs & 31;
-  if (R >= 32) {
-    // the run as a 128-bit number x3:x2:x1:x0 (the offsets are warp-uniform)
-    uint32_t x0, x1 = 0u, x2 = 0u, x3 = 0u;
-    if constexpr (sizeof(T) == 4) {
-      x0 = v[0];
-      place32(v[1], ln, x0, x1, x2, x3);
-      place32(v[2], 2 * ln, x0, x1, x2, x3);
-      place32(v[3], 3 * ln, x0, x1, x2, x3);
-    } else {
-      const uint32_t a0 = static_cast<uint32_t>(v[0]), a1 = static_cast<uint32_t>(v[0] >> 32);
-      const uint32_t b0 = static_cast<uint32_t>(v[1]), b1 = static_cast<uint32_t>(v[1] >> 32);
-      if (ln >= 32) {
-        const int r = ln - 32;
-        x0 = a0;
-        x1 = a1 | (b0 << r);
-        x2 = __funnelshift_l(b0, b1, r);
-        x3 = __funnelshift_l(b1, 0u, r);
-      } else {  // both values fit in 31 bits
-        x0 = a0 | (b0 << ln);
-        x1 = __funnelshift_l(b0, 0u, ln);
-      }
-    }
-    // shifted into place within the lane's first word
-    const uint32_t y0 = x0 << s;
-    const uint32_t y1 = __funnelshift_l(x0, x1, s);
-    const uint32_t y2 = __funnelshift_l(x1, x2, s);
-    const uint32_t y3 = __funnelshift_l(x2, x3, s);
-    const uint32_t y4 = __funnelshift_l(x3, 0u, s);
-    const int nfull = (s + R) >> 5;  // words 1 .. nfull-1 lie wholly in this run
-    const uint32_t tail = nfull == 1 ? y1 : (nfull == 2 ? y2 : (nfull == 3 ? y3 : y4));
-    // each word holds bits of at most two adjacent lanes: the next lane completes our tail
-    const uint32_t prev = __shfl_up_sync(0xffffffffu, tail, 1);
-    uint32_t* const d = pw + w0;
-    d[0] = s ? (y0 | prev) : y0;
-    if (nfull > 1) d[1] = y1;
-    if (nfull > 2) d[2] = y2;
-    if (nfull > 3) d[3] = y3;
-  } else {
-    // short runs: several lanes share a word.  A run of R < 32 bits starts in
-    // every word, so the lane whose run starts first in a word stores it
-    // plainly (no clearing pass); the other lanes, and the spill of each run
-    // into the next word, OR in after that store.  Lane 31's run ends on a
-    // word boundary (32 R bits in all), so no spill leaves the packed area.
-    uint32_t run = 0;
-#pragma unroll
-    for (int k = 0; k < P; ++k) run |= static_cast<uint32_t>(v[k]) << (k * ln);
-    const uint64_t sh = static_cast<uint64_t>(run) << s;
-    const uint32_t lo = static_cast<uint32_t>(sh), hi = static_cast<uint32_t>(sh >> 32);
-    const bool first = lane == 0 || (((lane - 1) * R) >> 5) != w0;
-    if (first) pw[w0] = lo;
-    __syncwarp();
-    if (!first && lo) atomicOr(&pw[w0], lo);
-    if (hi) atomicOr(&pw[w0 + 1], hi);
-  }
-}
-
-// The lane's bit run of four 32-bit values of width ln (8 <= ln <= 31) as a
-// 128-bit number x3:x2:x1:x0, without branches.
-__device__ __forceinline__ void run_words(const uint32_t (&v)[4], int ln, uint32_t& x0, uint32_t& x1, uint32_t& x2,
-                                          uint32_t& x3)
-{
-  // pairs (v0 | v1 << ln) and (v2 | v3 << ln), each below 2^62; then the second
-  // pair shifted by 2 ln (16 .. 62) onto the first
-  const uint32_t a0 = v[0] | (v[1] << ln), a1 = __funnelshift_l(v[1], 0u, ln);
-  const uint32_t b0 = v[2] | (v[3] << ln), b1 = __funnelshift_l(v[3], 0u, ln);
-  const int k = 2 * ln;
-  const bool q = k >= 32;
-  const int r = k & 31;
-  const uint32_t t0 = b0 << r, t1 = __funnelshift_l(b0, b1, r), t2 = __funnelshift_l(b1, 0u, r);
-  x0 = a0 | (q ? 0u : t0);
-  x1 = a1 | (q ? t0 : t1);
-  x2 = q ? t1 : t2;
-  x3 = q ? t2 : 0u;
-}
-
-// Packs a warp's SPW subchunks (offsets wbase, widths lnu).  When every run is
-// short, or (32-bit values) every run is long (32 <= P*ln, ln below the value
-// width), or (64-bit values) every run is long with values of at most 31 bits,
-// the subchunks go through one straight-line sequence each, so their shuffles,
-// shifts and stores overlap; other widths take the per-subchunk path.
-// (For 64-bit values the branch-free long run costs more than the overlap saves:
-// measured -2 % on lossless f64, +3.5-6 % on f32.)
-constexpr int PACK_GROUP = 2;  // subchunks whose long runs are built and exchanged together
-
-template <typename T, int SPW>
-__device__ __forceinline__ void pack_subchunks(uint32_t* pw, const int (&wbase)[SPW], const int (&lnu)[SPW],
-                                               const T (&v)[SPW][16 / sizeof(T)], int lane)
-{
-  constexpr int P = 16 / static_cast<int>(sizeof(T));
-  constexpr int TB = 8 * static_cast<int>(sizeof(T));
-  bool all_long = sizeof(T) == 4, all_short = true, all_narrow = sizeof(T) == 8;
-#pragma unroll
-  for (int u = 0; u < SPW; ++u) {
-    all_long &= P * lnu[u] >= 32 && lnu[u] < TB;
-    all_short &= P * lnu[u] < 32;
-    all_narrow &= P * lnu[u] >= 32 && lnu[u] < 32;  // 64-bit values of 16 .. 31 bits
-  }
-  if (all_long) {
-    if constexpr (sizeof(T) == 4) {
-#pragma unroll
-      for (int g = 0; g < SPW; g += PACK_GROUP) {
-        uint32_t y[SPW][5], tl[SPW], pv[SPW];
-        int nf[SPW];
-#pragma unroll
-        for (int u = g; u < g + PACK_GROUP; ++u) {
-          const int R = P * lnu[u];
-          const int s = (lane * R) & 31;
-          uint32_t x0, x1, x2, x3;
-          run_words(v[u], lnu[u], x0, x1, x2, x3);
-          y[u][0] = x0 << s;
-          y[u][1] = __funnelshift_l(x0, x1, s);
-          y[u][2] = __funnelshift_l(x1, x2, s);
-          y[u][3] = __funnelshift_l(x2, x3, s);
-          y[u][4] = __funnelshift_l(x3, 0u, s);
-          nf[u] = (s + R) >> 5;
-          tl[u] = nf[u] == 1 ? y[u][1] : (nf[u] == 2 ? y[u][2] : (nf[u] == 3 ? y[u][3] : y[u][4]));
-        }
-#pragma unroll
-        for (int u = g; u < g + PACK_GROUP; ++u) pv[u] = __shfl_up_sync(0xffffffffu, tl[u], 1);
-#pragma unroll
-        for (int u = g; u < g + PACK_GROUP; ++u) {
-          const int rs = lane * P * lnu[u];
-          uint32_t* const d = pw + wbase[u] + (rs >> 5);
-          d[0] = (rs & 31) ? (y[u][0] | pv[u]) : y[u][0];
-          if (nf[u] > 1) d[1] = y[u][1];
-          if (nf[u] > 2) d[2] = y[u][2];
-          if (nf[u] > 3) d[3] = y[u][3];
-        }
-      }
-    }
-  } else if (all_short) {
-    // see pack_subchunk: the first run in each word stores it, the rest OR in
-    uint32_t lo[SPW], hi[SPW];
-    int w[SPW];
-    bool first[SPW];
-#pragma unroll
-    for (int u = 0; u < SPW; ++u) {
-      const int ln = lnu[u];
-      const int R = P * ln;
-      uint32_t run = 0;
-#pragma unroll
-      for (int k = 0; k < P; ++k) run |= static_cast<uint32_t>(v[u][k]) << (k * ln);
-      const uint64_t sh = static_cast<uint64_t>(run) << ((lane * R) & 31);
-      lo[u] = static_cast<uint32_t>(sh);
-      hi[u] = static_cast<uint32_t>(sh >> 32);
-      w[u] = wbase[u] + ((lane * R) >> 5);
-      first[u] = ln != 0 && (lane == 0 || (((lane - 1) * R) >> 5) != ((lane * R) >> 5));
-      if (first[u]) pw[w[u]] = lo[u];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < SPW; ++u) {
-      if (!first[u] && lo[u]) atomicOr(&pw[w[u]], lo[u]);
-      if (hi[u]) atomicOr(&pw[w[u] + 1], hi[u]);
-    }
-  } else if (all_narrow) {
-    if constexpr (sizeof(T) == 8) {
-      // 64-bit values that fit in 31 bits (typical of lossy chunks): the lane's two
-      // values make a run of 32 .. 62 bits, two words before the shift and at most
-      // three after it, built from the low halves only
-      uint32_t y0[SPW], y1[SPW], tl[SPW], pv[SPW];
-      int nf[SPW];
-#pragma unroll
-      for (int u = 0; u < SPW; ++u) {
-        const int ln = lnu[u];
-        const int R = P * ln;
-        const int sh = (lane * R) & 31;
-        const uint32_t a0 = static_cast<uint32_t>(v[u][0]), b0 = static_cast<uint32_t>(v[u][1]);
-        const uint32_t x0 = a0 | (b0 << ln), x1 = __funnelshift_l(b0, 0u, ln);
-        y0[u] = x0 << sh;
-        y1[u] = __funnelshift_l(x0, x1, sh);
-        const uint32_t y2 = __funnelshift_l(x1, 0u, sh);
-        nf[u] = (sh + R) >> 5;
-        tl[u] = nf[u] == 1 ? y1[u] : y2;
-      }
-#pragma unroll
-      for (int u = 0; u < SPW; ++u) pv[u] = __shfl_up_sync(0xffffffffu, tl[u], 1);
-#pragma unroll
-      for (int u = 0; u < SPW; ++u) {
-        const int rs = lane * P * lnu[u];
-        uint32_t* const d = pw + wbase[u] + (rs >> 5);
-        d[0] = (rs & 31) ? (y0[u] | pv[u]) : y0[u];
-        if (nf[u] > 1) d[1] = y1[u];
-      }
-    }
-  } else {
-#pragma unroll
-    for (int u = 0; u < SPW; ++u) pack_subchunk<T>(pw + wbase[u], lnu[u], v[u], lane);
-  }
-}
-
-
-// The per-chunk work of a compute warp, in three steps shared by both encode
-// kernels.  KIND: bit 0 = 64-bit values, bit 1 = lossy.
-template <int KIND>
-using EncVal = typename std::conditional<(KIND & 1) != 0, uint64_t, uint32_t>::type;
-
-// Phase A: the warp's subchunks cw, cw + CW, ... of the staged chunk into
-// registers, transformed or quantized, and their bit widths into lnv (the stage
-// always holds a full 16 KB chunk: partial chunks are zero padded).
-template <int KIND, class S>
-__device__ __forceinline__ void chunk_phase_a(const uint8_t* stg, const QParams& q, int* lnv, int cw, int lane,
-                                              EncVal<KIND> (&vals)[S::SPW][16 / sizeof(EncVal<KIND>)])
-{
-  using T = EncVal<KIND>;
-  constexpr bool LOSSY = (KIND & 2) != 0;
-  constexpr int P = 16 / static_cast<int>(sizeof(T));
-#pragma unroll
-  for (int u = 0; u < S::SPW; ++u) {
-    const int i = cw + u * S::CW;
-    const uint4 w4 = *reinterpret_cast<const uint4*>(stg + i * 512 + lane * 16);
-    if constexpr (sizeof(T) == 4) {
-      vals[u][0] = w4.x; vals[u][1] = w4.y; vals[u][2] = w4.z; vals[u][3] = w4.w;
-    } else {
-      vals[u][0] = (static_cast<uint64_t>(w4.y) << 32) | w4.x;
-      vals[u][1] = (static_cast<uint64_t>(w4.w) << 32) | w4.z;
-    }
-    T orv = 0;
-#pragma unroll
-    for (int p = 0; p < P; ++p) {
-      vals[u][p] = encode_value<LOSSY>(vals[u][p], q);
-      orv |= vals[u][p];
-    }
-    const int w = warp_bit_width(orv);
-    if (lane == 0) lnv[i] = w;
-  }
-}
-
-// The chunk's packed words (wtot) and its size in the stream (compressed iff
-// 34 + 4 wtot < osize), from every subchunk's width (all lanes, any warp).
-struct ChunkSize {
-  int ln;    // width of subchunk `lane`
-  int wc;    // 32-bit words of subchunk `lane`
-  int wtot;  // packed words of the chunk
-  int csize;
-  bool comp;
-};
-template <typename T>
-__device__ __forceinline__ ChunkSize chunk_size(const int* lnv, int lane, int osize)
-{
-  using V = VT<T>;
-  ChunkSize z;
-  z.ln = lnv[lane];
-  z.wc = (V::VPS * z.ln) >> 5;
-  // totals by warp reductions (independent, no shuffle-scan chain)
-  z.wtot = __reduce_add_sync(0xffffffffu, z.wc);
-  const int newsize = 34 + 4 * z.wtot;
-  z.comp = newsize < osize;
-  z.csize = z.comp ? newsize : osize;
-  return z;
-}
-
-// Packs a compressible chunk from registers to `dst` (16-byte aligned): the 32
-// width bytes, the packed words, the int16 trailer.
-template <int KIND, class S>
-__device__ __forceinline__ void chunk_pack(uint8_t* dst, const ChunkSize& z, int osize, int cw, int lane,
-                                           const EncVal<KIND> (&vals)[S::SPW][16 / sizeof(EncVal<KIND>)])
-{
-  using T = EncVal<KIND>;
-  uint32_t* const pw = reinterpret_cast<uint32_t*>(dst + 32);
-  int wbase[S::SPW], lnu[S::SPW];  // all offsets and widths first: the reductions overlap
-#pragma unroll
-  for (int u = 0; u < S::SPW; ++u) {
-    const int i = cw + u * S::CW;
-    wbase[u] = __reduce_add_sync(0xffffffffu, lane < i ? z.wc : 0);  // words of subchunks before i
-    lnu[u] = __shfl_sync(0xffffffffu, z.ln, i);
-  }
-  pack_subchunks<T, S::SPW>(pw, wbase, lnu, vals, lane);
-  if (cw == 0) {
-    dst[lane] = static_cast<uint8_t>(z.ln);
-    if (lane == 0) *reinterpret_cast<int16_t*>(dst + 32 + 4 * z.wtot) = static_cast<int16_t>(osize);
-  }
-}
-
-// Transform, size, publish and pack one chunk in place (compute warps of
-// k_encode).  The barrier after phase A is the compute warps' only CTA barrier
-// per chunk and their point of agreement: every warp arrives there, with `skip`
-// (no chunk: the end, or a failed wait) and `fail` (this thread's wait gave up);
-// returns 2 if any thread failed, 1 at the end, 0 when the chunk was processed.
-template <int KIND, class S>
-__device__ __forceinline__ int compute_chunk(uint8_t* stg, EncMeta& me, EncMisc<S::ST>& m, uint64_t* flags, int cw,
-                                             int lane, int tid, int par, bool skip, bool fail)
-{
-  using T = EncVal<KIND>;
-  int* const lnv = m.lnv[par];
-  T vals[S::SPW][16 / sizeof(T)];
-  if (!skip) chunk_phase_a<KIND, S>(stg, me.q, lnv, cw, lane, vals);
-  if (cbar_or<S::CW>(fail)) return 2;
-  if (skip) return 1;
-  const int osize = me.osize;
-  const ChunkSize z = chunk_size<T>(lnv, lane, osize);
-  if (tid == 0) {
-    const int s = static_cast<int>(&me - m.meta);
-    me.csize = z.csize;
-    me.comp = z.comp;
-    st_relaxed_u64(&flags[me.g], (me.c == 0 ? FLAG_INC : FLAG_AGG) | static_cast<uint64_t>(z.csize));
-    mbar_arrive(&m.sized[s]);
-  }
-  if (z.comp) chunk_pack<KIND, S>(stg, z, osize, cw, lane, vals);
-  return 0;
-}
-
-// Chunk sources: one buffer (the plain entry points) or a table of buffers (the
-// batched entry points; every chunk of every buffer is one ticket).
-template <bool BATCH>
-struct EncSource;
-
-template <>
-struct EncSource<false> {
-  const EncArgs& a;
-  long long chunks;
-  __device__ long long total() const { return chunks; }
-  // fills the chunk's description; returns its first byte
-  __device__ const uint8_t* describe(long long g, EncMeta& me, int kind) const
-  {
-    me.g = g;
-    me.c = g;
-    me.seg = 0;
-    me.chunks = chunks;
-    me.insize = a.insize;
-    me.out = a.out;
-    me.outsize = a.outsize;
-    me.q = a.q;
-    me.kind = kind;
-    me.osize = static_cast<int>(min(static_cast<long long>(CS), a.insize - g * CS));
-    return a.in + g * CS;
-  }
-};
-
-template <>
-struct EncSource<true> {
-  const BatchEncArgs& a;
-  const long long* cb;  // shared memory: first chunk id of each job, then the total
-  __device__ long long total() const { return cb[a.njobs]; }
-  __device__ const uint8_t* describe(long long g, EncMeta& me, int) const
-  {
-    int lo = 0, hi = a.njobs - 1;  // last job whose first chunk id is <= g (empty jobs are skipped)
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (cb[mid] <= g) lo = mid;
-      else hi = mid - 1;
-    }
-    const BatchJob& j = a.jobs[lo];
-    const long long c = g - cb[lo];
-    me.g = g;
-    me.c = c;
-    me.seg = cb[lo];
-    me.chunks = j.chunks;
-    me.insize = j.insize;
-    me.out = j.out;
-    me.outsize = j.outsize;
-    me.q = j.q;
-    me.kind = j.kind;
-    me.osize = static_cast<int>(min(static_cast<long long>(CS), j.insize - c * CS));
-    return j.in + c * CS;
-  }
-};
-
-template <int KIND, bool BATCH, class S>
-__global__ void __launch_bounds__(S::NT, S::MINB) k_encode(const typename std::conditional<BATCH, BatchEncArgs, EncArgs>::type a)
-{
-  constexpr int ENC_STAGES = S::ST;
-  constexpr int ENC_AHEAD = S::AHEAD;
-  constexpr int ENC_CW = S::CW;
-  constexpr int ENC_NT = S::NT;
-  extern __shared__ __align__(128) uint8_t smem[];
-  uint8_t* const stage0 = smem;
-  EncMisc<ENC_STAGES>& m = *reinterpret_cast<EncMisc<ENC_STAGES>*>(smem + ENC_STAGES * STAGE_BYTES);
-  long long* const cb = reinterpret_cast<long long*>(smem + enc_smem<S>());
-
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  // this launch's counter block and flag region: alternating by epoch in the
-  // single-buffer form (self-resetting workspace), block 0 and the first region
-  // of a workspace cleared before each run in the batched form
-  const WsPhase ph = [&]() {
-    if constexpr (BATCH) return WsPhase::fixed(a.ws);
-    else return WsPhase::of(a.ws, a.flag_cap);
-  }();
-  uint64_t* const hdr = ph.hdr;
-  uint64_t* const flags = ph.flags;
-
-  if constexpr (BATCH) {
-    for (int i = tid; i <= a.njobs; i += ENC_NT) cb[i] = a.chunk_base[i];
-  }
-  if (tid == 0) {
-    for (int s = 0; s < ENC_STAGES; ++s) {
-      mbar_init(&m.full[s], 1);
-      mbar_init(&m.sized[s], 1);
-      mbar_init(&m.placed[s], 1);
-      mbar_init(&m.packed[s], ENC_CW);  // one arrival per compute warp
-    }
-    mbar_fence_init();
-  }
-  // the producer's first ticket, taken while the barriers are set up (the
-  // counter was reset by the previous launch's last CTA)
-  long long first_ticket = NO_CHUNK;
-  if (warp == ENC_CW && lane == 0)
-    first_ticket = static_cast<long long>(atomicAdd(reinterpret_cast<unsigned long long*>(&a.ws[WS_TICKET]), 1ull));
-  __syncthreads();
-
-  EncSource<BATCH> src = [&]() {
-    if constexpr (BATCH) return EncSource<true>{a, cb};
-    else return EncSource<false>{a, (a.insize + CS - 1) / CS};
-  }();
-  const long long total = src.total();
-
-  if (warp == ENC_CW) {
-    // ============ producer warp: tickets, TMA copies and the chunks' stores ============
-    // Tickets are taken just before their chunk's copy is issued, never earlier:
-    // a ticket held long before its chunk is processed makes every later chunk's
-    // look-back wait for it.  The stage's previous chunk is stored to the stream by
-    // this warp right before the stage is refilled, so the compute warps go from
-    // one chunk's pack straight to the next chunk's transform.
-    unsigned long long* const tick = reinterpret_cast<unsigned long long*>(&a.ws[WS_TICKET]);
-    // stores chunk q (stage q % ENC_STAGES) once it is packed and placed
-    auto store_q = [&](int q) -> bool {
-      const int sq = q % ENC_STAGES;
-      const uint32_t pq = (q / ENC_STAGES) & 1;
-      if (!mbar_wait_bounded(&m.packed[sq], pq)) return false;
-      if (!mbar_wait_bounded(&m.placed[sq], pq)) return false;
-      const EncMeta& me = m.meta[sq];
-      const long long excl = me.excl;
-      if (excl >= 0) {
-        uint8_t* const out = me.out;
-        store_shifted<32>(out + 8 + 2 * me.chunks + excl, stage0 + sq * STAGE_BYTES, me.csize, lane);
-        if (lane == 0) *reinterpret_cast<uint16_t*>(out + 8 + 2 * me.c) = static_cast<uint16_t>(me.csize);
-      }
-      // the stage's generic accesses are ordered before the TMA write that refills it
-      fence_proxy_async_smem();
-      __syncwarp();
-      return true;
-    };
-    unsigned issued = 0;      // stages whose last use was a TMA copy (lane 0's view)
-    unsigned issued_par = 0;  // parity of that use
-    bool more = true;
-    for (int seq = 0;; ++seq) {
-      const int s = seq % ENC_STAGES;
-      bool ok = true;
-      if (seq >= ENC_AHEAD)
-        ok = mbar_wait_bounded(&m.sized[(seq - ENC_AHEAD) % ENC_STAGES], ((seq - ENC_AHEAD) / ENC_STAGES) & 1);
-      if (ok && seq >= ENC_STAGES) ok = store_q(seq - ENC_STAGES);
-      if (__any_sync(0xffffffffu, !ok)) {
-        if (lane == 0) set_status(hdr, ST_TIMEOUT, -1);
-        break;
-      }
-      long long t = NO_CHUNK;
-      if (lane == 0 && more) t = seq == 0 ? first_ticket : static_cast<long long>(atomicAdd(tick, 1ull));
-      t = __shfl_sync(0xffffffffu, t, 0);
-      uint8_t* const stg = stage0 + s * STAGE_BYTES;
-      EncMeta& me = m.meta[s];
-      if (t < total) {
-        const uint8_t* in = nullptr;
-        if (lane == 0) in = src.describe(t, me, KIND);
-        __syncwarp();
-        in = reinterpret_cast<const uint8_t*>(__shfl_sync(0xffffffffu, reinterpret_cast<uintptr_t>(in), 0));
-        const int osize = me.osize;
-        if ((reinterpret_cast<uintptr_t>(in) & 15u) == 0u && osize == CS) {
-          if (lane == 0) {
-            mbar_arrive_expect_tx(&m.full[s], CS);
-            tma_load_1d(stg, in, CS, &m.full[s]);
-            issued |= 1u << s;
-            issued_par = (issued_par & ~(1u << s)) | (((seq / ENC_STAGES) & 1u) << s);
-          }
-        } else {
-          // last partial chunk or an input that is not 16-byte aligned: 4-byte
-          // loads (inputs are at least 4-byte aligned), zero padding up to the full
-          // chunk (the padding is encoded too)
-          const uint32_t* const gin = reinterpret_cast<const uint32_t*>(in);
-          uint32_t* const sv = reinterpret_cast<uint32_t*>(stg);
-          constexpr int U = 16;  // independent loads in flight per lane
-          for (int k0 = 0; k0 < CS / 4; k0 += 32 * U) {
-            uint32_t v[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              const int k = k0 + u * 32 + lane;
-              v[u] = 4 * k < osize ? gin[k] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) sv[k0 + u * 32 + lane] = v[u];
-          }
-          __syncwarp();
-          if (lane == 0) {
-            issued &= ~(1u << s);
-            mbar_arrive(&m.full[s]);  // release: the stores above are visible to its waiters
-          }
-        }
-      } else {
-        more = false;
-        if (lane == 0) {
-          me.g = NO_CHUNK;
-          issued &= ~(1u << s);
-          mbar_arrive(&m.full[s]);
-        }
-      }
-      if (!more) break;
-    }
-    // (the chunks still in stages, the last ENC_STAGES - 1, are stored by the
-    // compute warps, idle by then: eight warps instead of one at the kernel's end)
-    // never leave with a bulk copy still landing in this CTA's shared memory
-    if (lane == 0) {
-      for (int s = 0; s < ENC_STAGES; ++s)
-        if (issued & (1u << s)) mbar_wait_bounded(&m.full[s], (issued_par >> s) & 1u);
-    }
-  } else if (warp == ENC_CW + 1) {
-    // ===================== scanner warp: decoupled look-back =====================
-    if constexpr (!BATCH) ph.clear_other_share(lane);
-    for (int seq = 0;; ++seq) {
-      const int s = seq % ENC_STAGES;
-      const uint32_t par = (seq / ENC_STAGES) & 1;
-      bool ok = mbar_wait_bounded(&m.full[s], par);
-      if (__any_sync(0xffffffffu, !ok)) break;  // the compute warps report it
-      EncMeta& me = m.meta[s];
-      const long long g = me.g;
-      if (g == NO_CHUNK) break;
-      // The look-back needs only the predecessors' sizes, so it starts as soon as
-      // the chunk has landed and overlaps the compute warps' phase A (measured
-      // against starting once the chunk is sized: +1-6 %).
-      const long long c = me.c;
-      long long excl = 0;
-      unsigned err = 0;
-      if (c > 0) {
-        excl = lookback(flags, g, me.seg, hdr);
-        if (excl < 0) err = ST_TIMEOUT;
-        else if (excl > c * CS) err = ST_CAPACITY;
-        if (err) excl = -1;
-      }
-      ok = mbar_wait_bounded(&m.sized[s], par);
-      if (__any_sync(0xffffffffu, !ok)) {
-        if (lane == 0) set_status(hdr, ST_TIMEOUT, g);
-        break;
-      }
-      const int csize = me.csize;
-      if (lane == 0) {
-        if (c > 0) {
-          if (err) set_status(hdr, err, g);
-          // an impossible prefix is replaced by the largest legal one so that
-          // every later chunk still writes inside the output bound
-          st_relaxed_u64(&flags[g], FLAG_INC | static_cast<uint64_t>(excl >= 0 ? excl + csize : (c + 1) * CS));
-        }
-        me.excl = excl;
-        if (c == me.chunks - 1 && excl >= 0) {
-          if constexpr (BATCH) {  // the buffer is complete: its header and size
-            *reinterpret_cast<long long*>(me.out) = me.insize;
-            *me.outsize = 8 + 2 * me.chunks + excl + csize;
-          } else {
-            hdr[WS_TOTAL] = static_cast<uint64_t>(excl + csize);
-          }
-        }
-        mbar_arrive(&m.placed[s]);
-      }
-    }
-  } else {
-    // ===================== compute warps =====================
-    // Warps pass each other freely between the barriers of compute_chunk: each
-    // waits for its stage itself, and a stage goes back to the producer warp once
-    // every compute warp has packed its share of the chunk.
-    const int cw = warp;
-    bool late = false;  // a wait of this thread gave up
-    int seq = 0;
-    int r = 0;
-    for (;; ++seq) {
-      const int s = seq % ENC_STAGES;
-      if (!mbar_wait_bounded(&m.full[s], (seq / ENC_STAGES) & 1)) {
-        if (lane == 0) set_status(hdr, ST_TIMEOUT, -1);
-        late = true;
-      }
-      EncMeta& me = m.meta[s];
-      // warp-uniform: phase A's warp collectives need every lane or none
-      const bool wlate = __any_sync(0xffffffffu, late);
-      const bool skip = wlate || me.g == NO_CHUNK;
-      uint8_t* const stg = stage0 + s * STAGE_BYTES;
-      if constexpr (KIND >= 0) {
-        r = compute_chunk<KIND, S>(stg, me, m, flags, cw, lane, tid, seq & 1, skip, wlate);
-      } else {
-        switch (skip ? 0 : me.kind) {
-          case 0: r = compute_chunk<0, S>(stg, me, m, flags, cw, lane, tid, seq & 1, skip, wlate); break;
-          case 1: r = compute_chunk<1, S>(stg, me, m, flags, cw, lane, tid, seq & 1, skip, wlate); break;
-          case 2: r = compute_chunk<2, S>(stg, me, m, flags, cw, lane, tid, seq & 1, skip, wlate); break;
-          default: r = compute_chunk<3, S>(stg, me, m, flags, cw, lane, tid, seq & 1, skip, wlate); break;
-        }
-      }
-      if (r != 0) break;  // end of the work (1) or a wait that gave up (2)
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&m.packed[s]);
-    }
-    if (r == 1) {
-      // The producer stored chunks 0 .. seq - ENC_STAGES as it refilled their
-      // stages (seq is the end marker); the rest, packed before the end's
-      // barrier, are stored here once placed.
-      for (int q = seq >= ENC_STAGES - 1 ? seq - ENC_STAGES + 1 : 0; q < seq; ++q) {
-        const int sq = q % ENC_STAGES;
-        if (!mbar_wait_bounded(&m.placed[sq], (q / ENC_STAGES) & 1)) {
-          if (lane == 0) set_status(hdr, ST_TIMEOUT, -1);
-          continue;
-        }
-        const EncMeta& me = m.meta[sq];
-        const long long excl = me.excl;
-        if (excl >= 0) {
-          store_shifted<ENC_CW * 32>(me.out + 8 + 2 * me.chunks + excl, stage0 + sq * STAGE_BYTES, me.csize, tid);
-          if (tid == 0) *reinterpret_cast<uint16_t*>(me.out + 8 + 2 * me.c) = static_cast<uint16_t>(me.csize);
-        }
-      }
-    }
-  }
-
-  // ---- epilogue: the last CTA out finishes the outputs -----------------------
-  __syncthreads();
-  __shared__ int last_cta;
-  if (tid == 0) {
-    __threadfence();
-    const unsigned long long d = atomicAdd(reinterpret_cast<unsigned long long*>(&a.ws[WS_DONE]), 1ull);
-    last_cta = d == gridDim.x - 1;
-    if (last_cta) __threadfence();
-  }
-  __syncthreads();
-  if (last_cta) {
-    const unsigned long long st = ld_relaxed_u64(&hdr[WS_STATUS]);
-    if constexpr (BATCH) {
-      // buffers without chunks get their header-only stream; an error anywhere
-      // turns every size into -status
-      for (int i = tid; i < a.njobs; i += ENC_NT) {
-        const BatchJob& j = a.jobs[i];
-        if (st) {
-          *j.outsize = -static_cast<long long>(st);
-        } else if (j.chunks == 0) {
-          *reinterpret_cast<long long*>(j.out) = 0;
-          *j.outsize = 8;
-        }
-      }
-    } else if (tid == 0) {
-      const long long chunks = (a.insize + CS - 1) / CS;
-      const long long tot = chunks ? static_cast<long long>(ld_relaxed_u64(&hdr[WS_TOTAL])) : 0ll;
-      *reinterpret_cast<long long*>(a.out) = a.insize;
-      *a.outsize = st ? -static_cast<long long>(st) : 8 + 2 * chunks + tot;
-      ph.finish(a.ws, chunks);
-    }
-  }
-}
 
 // ============================================================================
 // decode
@@ -1178,6 +394,7 @@ __global__ void __launch_bounds__(NT, MINB) k_decode(const DecArgs a)
 // batched decode: a prepass places every chunk, then a persistent kernel with a
 // producer warp and 8 compute warps decodes chunks in any order
 // ============================================================================
+constexpr long long NO_CHUNK = 0x7fffffffffffffffll;
 constexpr int DB_STAGES = 4;
 constexpr int DB_CW = 8;
 constexpr int DB_NT = (DB_CW + 1) * 32;
@@ -1411,20 +628,6 @@ __global__ void __launch_bounds__(DB_NT, DB_MINB) k_decode_batch(const BatchDecA
 // ============================================================================
 // launchers
 // ============================================================================
-// Sets the dynamic shared memory limit of `k` once per device.
-template <typename K>
-static cudaError_t ensure_smem_attr(K k, int bytes, unsigned long long* done_mask)
-{
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (__atomic_load_n(done_mask, __ATOMIC_ACQUIRE) & bit) return cudaSuccess;
-  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) __atomic_fetch_or(done_mask, bit, __ATOMIC_RELEASE);
-  return e;
-}
-
 // Decode launch shapes: threads per CTA and the CTAs per SM the registers are
 // budgeted for (index = the C ABI's shape number).
 template <int NT_, int MINB_>
@@ -1436,28 +639,6 @@ using DecShape0 = DecShape<256, 4>;  // default
 using DecShape1 = DecShape<128, 6>;
 using DecShape2 = DecShape<512, 2>;
 constexpr int DEC_SHAPES = 3;
-
-template <int KIND, class S>
-static cudaError_t launch_enc_k(const EncArgs& a, int grid, cudaStream_t st)
-{
-  auto k = k_encode<KIND, false, S>;
-  static unsigned long long attr = 0;
-  cudaError_t e = ensure_smem_attr(k, enc_smem<S>(), &attr);
-  if (e != cudaSuccess) return e;
-  k<<<grid, S::NT, enc_smem<S>(), st>>>(a);
-  return cudaGetLastError();
-}
-
-template <int KIND, class S>
-static int enc_occupancy()
-{
-  auto k = k_encode<KIND, false, S>;
-  // the smem attribute must be set before the occupancy query counts dynamic smem
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, enc_smem<S>());
-  int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, S::NT, enc_smem<S>());
-  return n;
-}
 
 template <typename T, bool LOSSY, class S>
 static cudaError_t launch_dec_k(const DecArgs& a, int grid, cudaStream_t st)
@@ -1480,30 +661,6 @@ static int dec_occupancy()
   return n;
 }
 
-template <int KIND>
-static cudaError_t launch_enc_kind(int shape, const EncArgs& a, int grid, cudaStream_t st)
-{
-  switch (shape) {
-    case 1: return launch_enc_k<KIND, EncShape1>(a, grid, st);
-    case 2: return launch_enc_k<KIND, EncShape2>(a, grid, st);
-    case 3: return launch_enc_k<KIND, EncShape3>(a, grid, st);
-    case 4: return launch_enc_k<KIND, EncShape4>(a, grid, st);
-    default: return launch_enc_k<KIND, EncShape0>(a, grid, st);
-  }
-}
-
-template <int KIND>
-static int enc_occupancy_kind(int shape)
-{
-  switch (shape) {
-    case 1: return enc_occupancy<KIND, EncShape1>();
-    case 2: return enc_occupancy<KIND, EncShape2>();
-    case 3: return enc_occupancy<KIND, EncShape3>();
-    case 4: return enc_occupancy<KIND, EncShape4>();
-    default: return enc_occupancy<KIND, EncShape0>();
-  }
-}
-
 template <typename T, bool LOSSY>
 static cudaError_t launch_dec_kind(int shape, const DecArgs& a, int grid, cudaStream_t st)
 {
@@ -1524,12 +681,6 @@ static int dec_occupancy_kind(int shape)
   }
 }
 
-cudaError_t launch_encode(int width, bool lossy, int shape, const EncArgs& a, int grid, cudaStream_t st)
-{
-  if (width == 4) return lossy ? launch_enc_kind<2>(shape, a, grid, st) : launch_enc_kind<0>(shape, a, grid, st);
-  return lossy ? launch_enc_kind<3>(shape, a, grid, st) : launch_enc_kind<1>(shape, a, grid, st);
-}
-
 cudaError_t launch_decode(int width, bool lossy, int shape, const DecArgs& a, int grid, cudaStream_t st)
 {
   if (width == 4)
@@ -1539,47 +690,22 @@ cudaError_t launch_decode(int width, bool lossy, int shape, const DecArgs& a, in
 
 int blocks_per_sm(int width, bool lossy, bool enc, int shape)
 {
-  if (enc) {
-    if (width == 4) return lossy ? enc_occupancy_kind<2>(shape) : enc_occupancy_kind<0>(shape);
-    return lossy ? enc_occupancy_kind<3>(shape) : enc_occupancy_kind<1>(shape);
-  }
+  if (enc) return encode_blocks_per_sm(width, lossy, shape);
   if (width == 4) return lossy ? dec_occupancy_kind<uint32_t, true>(shape) : dec_occupancy_kind<uint32_t, false>(shape);
   return lossy ? dec_occupancy_kind<uint64_t, true>(shape) : dec_occupancy_kind<uint64_t, false>(shape);
 }
 
 ShapeInfo shape_info(bool enc, int shape)
 {
-  ShapeInfo r{};
-  if (enc) {
-    switch (shape) {
-      case 1: r = {EncShape1::NT, EncShape1::CW, EncShape1::ST, EncShape1::MINB}; break;
-      case 2: r = {EncShape2::NT, EncShape2::CW, EncShape2::ST, EncShape2::MINB}; break;
-      case 3: r = {EncShape3::NT, EncShape3::CW, EncShape3::ST, EncShape3::MINB}; break;
-      case 4: r = {EncShape4::NT, EncShape4::CW, EncShape4::ST, EncShape4::MINB}; break;
-      default: r = {EncShape0::NT, EncShape0::CW, EncShape0::ST, EncShape0::MINB}; break;
-    }
-  } else {
-    switch (shape) {
-      case 1: r = {DecShape1::NT, DecShape1::NT / 32, DEC_STAGES, DecShape1::MINB}; break;
-      case 2: r = {DecShape2::NT, DecShape2::NT / 32, DEC_STAGES, DecShape2::MINB}; break;
-      default: r = {DecShape0::NT, DecShape0::NT / 32, DEC_STAGES, DecShape0::MINB}; break;
-    }
+  if (enc) return encode_shape_info(shape);
+  switch (shape) {
+    case 1: return {DecShape1::NT, DecShape1::NT / 32, DEC_STAGES, DecShape1::MINB};
+    case 2: return {DecShape2::NT, DecShape2::NT / 32, DEC_STAGES, DecShape2::MINB};
+    default: return {DecShape0::NT, DecShape0::NT / 32, DEC_STAGES, DecShape0::MINB};
   }
-  return r;
 }
 
-int shape_count(bool enc) { return enc ? ENC_SHAPES : DEC_SHAPES; }
-
-cudaError_t launch_encode_batch(const BatchEncArgs& a, int grid, cudaStream_t st)
-{
-  using S = EncShape0;
-  auto k = k_encode<-1, true, S>;
-  static unsigned long long attr = 0;
-  cudaError_t e = ensure_smem_attr(k, enc_batch_smem<S>(), &attr);
-  if (e != cudaSuccess) return e;
-  k<<<grid, S::NT, enc_batch_smem<S>(), st>>>(a);
-  return cudaGetLastError();
-}
+int shape_count(bool enc) { return enc ? encode_shape_count() : DEC_SHAPES; }
 
 cudaError_t launch_decode_batch(const BatchDecArgs& a, int grid, cudaStream_t st)
 {
@@ -1598,15 +724,6 @@ int decode_batch_blocks_per_sm()
   cudaFuncSetAttribute(k_decode_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, DB_SMEM);
   int n = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_decode_batch, DB_NT, DB_SMEM);
-  return n;
-}
-
-int encode_batch_blocks_per_sm()
-{
-  using S = EncShape0;
-  cudaFuncSetAttribute(k_encode<-1, true, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, enc_batch_smem<S>());
-  int n = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_encode<-1, true, S>, S::NT, enc_batch_smem<S>());
   return n;
 }
 

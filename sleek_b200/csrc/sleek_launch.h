@@ -25,7 +25,7 @@ struct EncArgs {
   uint8_t* out;          // device stream, >= upper bound size, 8-byte aligned
   long long* outsize;    // device: stream bytes, or -status on a device-detected error
   uint64_t* ws;          // workspace: header words + flag regions (self-resetting, see WsPhase)
-  long long flag_cap;    // flags per region (at least one per chunk)
+  long long flag_cap;    // words per region (at least one per chunk)
   QParams q;
 };
 
@@ -59,7 +59,8 @@ struct BatchEncArgs {
   const BatchJob* jobs;         // device table
   const long long* chunk_base;  // device: first chunk id of each job, then the total (njobs + 1)
   int njobs;
-  uint64_t* ws;                 // zeroed workspace: header words + one flag per chunk
+  uint64_t* ws;                 // zeroed workspace: header words + one word per chunk
+  uint64_t* starts;             // zeroed workspace: one word per job (the prefix before its first chunk)
 };
 
 struct BatchDecArgs {
@@ -72,11 +73,11 @@ struct BatchDecArgs {
   long long* actual_insize;     // workspace: bytes each stream decodes to
 };
 
-// Launch shapes of the single-buffer kernels (sleek_kernels.cu: EncShape*,
-// DecShape*); shape 0 is the default.  Every shape produces the same bytes.
+// Launch shapes of the single-buffer kernels (sleek_encode.cu: EncShape*,
+// sleek_kernels.cu: DecShape*); shape 0 is the default.  Every shape produces the same bytes.
 struct ShapeInfo {
   int threads;        // per CTA
-  int warps;          // compute warps (encode) / warps (decode)
+  int warps;          // warps that work on chunks
   int stages;         // shared-memory chunk stages
   int ctas_per_sm;    // CTAs per SM the registers are budgeted for
 };
@@ -85,6 +86,9 @@ ShapeInfo shape_info(bool enc, int shape);
 cudaError_t launch_encode(int width, bool lossy, int shape, const EncArgs& a, int grid, cudaStream_t st);
 cudaError_t launch_decode(int width, bool lossy, int shape, const DecArgs& a, int grid, cudaStream_t st);
 int blocks_per_sm(int width, bool lossy, bool enc, int shape);
+int encode_shape_count();
+ShapeInfo encode_shape_info(int shape);
+int encode_blocks_per_sm(int width, bool lossy, int shape);
 cudaError_t launch_decode_batch(const BatchDecArgs& a, int grid, cudaStream_t st);
 int decode_batch_blocks_per_sm();
 cudaError_t launch_encode_batch(const BatchEncArgs& a, int grid, cudaStream_t st);
