@@ -6,7 +6,7 @@
 // chunk ids, and uploads the job tables once; running it only clears the
 // workspace and launches (no host work, no allocation), so a run can be captured
 // in a CUDA graph and replayed.  Streams are bit-identical to the single-buffer
-// entry points (the batched look-back is segmented per buffer).
+// entry points (a chunk's place is relative to its buffer's first chunk).
 #include <cstdint>
 #include <cstring>
 #include <new>
@@ -263,9 +263,8 @@ int sleek_batch_plan_run(sleek_batch_plan* plan, void* d_workspace, size_t works
       a.chunk_base = g.d_cb;
       a.njobs = g.njobs;
       a.ws = ws;
-      a.offsets = reinterpret_cast<long long*>(ws + HDR_WORDS);
-      a.actual = a.offsets + g.chunks;
-      a.actual_insize = a.actual + g.njobs;
+      a.places = reinterpret_cast<unsigned long long*>(ws + HDR_WORDS);
+      a.actual = reinterpret_cast<long long*>(a.places + g.chunks);
       e = sleek::launch_decode_batch(a, grid_for(plan, g.chunks), st);
     } else {
       sleek::BatchEncArgs a;

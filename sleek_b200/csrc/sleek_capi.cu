@@ -2,7 +2,7 @@
 //
 // Host-side argument checks, grid sizing from the occupancy of the kernels on
 // the current device, workspace handling and error-bound derivation.  All
-// compute happens in sleek_encode.cu and sleek_kernels.cu; there is no CPU fallback.
+// compute happens in sleek_encode.cu and sleek_decode.cu; there is no CPU fallback.
 #include <cstdint>
 #include <cstring>
 #include <map>
@@ -79,7 +79,8 @@ int persistent_grid(int dev, int width, bool lossy, bool enc, long long bytes, i
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     d.sms = sms > 0 ? sms : 1;
   }
-  const Choice c = bytes < 0 ? Choice{} : d.choice[width == 8][lossy][enc][size_bucket(bytes)];
+  Choice c = bytes < 0 ? Choice{} : d.choice[width == 8][lossy][enc][size_bucket(bytes)];
+  if (c.shape == 0 && c.ctas == 0 && bytes >= 0) c.shape = sleek::default_shape(enc, (bytes + CS - 1) / CS, d.sms);
   int& b = d.bps[width == 8][lossy][enc][c.shape];
   if (b == 0) {
     const int n = sleek::blocks_per_sm(width, lossy, enc, c.shape);
@@ -123,7 +124,7 @@ int owned_workspace(int dev, cudaStream_t st, long long need_flags, OwnedWs* out
   return SLEEK_OK;
 }
 
-// The workspace of one single-buffer launch that uses `need_flags` look-back flags:
+// The workspace of one single-buffer launch that uses `need_flags` words besides the header:
 // the library-owned one of (device, stream) when user_ws is NULL (no clearing: it
 // resets itself), else the caller's, checked and cleared on `st` (epoch 0, so only
 // the first flag region is used).
@@ -208,7 +209,8 @@ int do_decompress(int width, bool lossy, sleek::QParams q, const unsigned char* 
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int shape = 0;
-  const int grid = persistent_grid(dev, width, lossy, false, out_cap >= 0 ? out_cap : in_len, &shape);
+  int grid = persistent_grid(dev, width, lossy, false, out_cap >= 0 ? out_cap : in_len, &shape);
+  if (out_cap >= 0 && grid > (out_cap + CS - 1) / CS) grid = out_cap > 0 ? static_cast<int>((out_cap + CS - 1) / CS) : 1;
   uint64_t* w = nullptr;
   long long cap = 0;
   rc = prepare_workspace(st, ws, wsb, grid, &w, &cap);

@@ -2,8 +2,8 @@
 //
 // Everything here is integer / bit arithmetic.  The value transforms restate the
 // reference's arithmetic exactly (that is what makes the byte stream identical);
-// the data movement (TMA bulk loads into shared memory, gather-form bit packing,
-// bounded decoupled look-back, 16-byte shifted stores) is this project's own.
+// the data movement (TMA bulk copies to and from shared memory, packing in place,
+// bounded waits for the chunks' places) is this project's own.
 #pragma once
 
 #include <cstdint>
@@ -15,15 +15,14 @@ namespace sleek {
 
 constexpr int CS = 16384;          // chunk bytes; fixed by the stream format
 constexpr int SC = 32;             // subchunks per chunk; fixed by the stream format
-constexpr int STAGE_BYTES = CS + 64;  // one chunk plus room for a 16-byte misaligned window
 
 // status codes shared with the C ABI (include/sleek_capi.h)
 constexpr unsigned ST_CORRUPT = 5;
 constexpr unsigned ST_TIMEOUT = 6;
 constexpr unsigned ST_CAPACITY = 9;
 
-// Workspace: 32 header words (u64 each), then the look-back flags.  Words 0 and
-// 1 are the launch's ticket and done counters; two blocks of per-launch results
+// Workspace: 32 header words (u64 each), then the chunks' sizes and their groups'
+// sums (ChunkScan).  Words 0 and 1 are the launch's ticket and done counters; two blocks of per-launch results
 // (status, total, error position, flags used) follow at words 0-7 and 8-15 (the
 // first block shares its first two words with the counters), then the launch
 // epoch (word 16) and words the range reduction uses (24-26).  Single-buffer
@@ -39,10 +38,9 @@ enum WsWord {
   WS_HDR_WORDS = 32
 };
 
-// look-back flag: state in bits 62-63, value in bits 0-61
-constexpr uint64_t FLAG_AGG = 1ull << 62;
-constexpr uint64_t FLAG_INC = 2ull << 62;
-constexpr uint64_t FLAG_VAL = (1ull << 62) - 1;
+// a published word whose value may be 0: bit 63 set, the value below
+constexpr uint64_t FLAG_SET = 1ull << 63;
+constexpr uint64_t FLAG_VAL = FLAG_SET - 1;
 
 constexpr unsigned long long SPIN_TIMEOUT_NS = 4000000000ull;  // 4 s of wall time per wait
 
@@ -54,13 +52,11 @@ template <> struct VT<uint32_t> {
   static constexpr int TB = 32;            // bits per value
   static constexpr int VPC = CS / 4;       // values per chunk
   static constexpr int VPS = VPC / SC;     // values per subchunk (128)
-  static constexpr int WPS_PER_LN = 2;     // packed u64 words per subchunk per bit of width
 };
 template <> struct VT<uint64_t> {
   static constexpr int TB = 64;
   static constexpr int VPC = CS / 8;
   static constexpr int VPS = VPC / SC;     // 64
-  static constexpr int WPS_PER_LN = 1;
 };
 
 // ----------------------------------------------------------------------------
@@ -168,18 +164,6 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void fence_proxy_async_smem()
 {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-__device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t* p)
-{
-  uint64_t v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void st_release_u64(uint64_t* p, uint64_t v)
-{
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 // Flags carry their own value, so publishing one needs no ordering against the
@@ -314,30 +298,31 @@ __device__ __forceinline__ uint64_t fwd(uint64_t x)
   return (static_cast<uint64_t>(th) << 32) | tl;
 }
 
-__device__ __forceinline__ uint32_t inv(uint32_t v)
+// The inverse, without branches.  With r the code rotated right by 1 (its lowest bit
+// on top): an odd code is the middle case's ~(2 w), so r = ~w and v = w + 2^24; an
+// even one is 2 v mod 2^32 with the bit that 2 v lost set exactly where the exponent
+// field is not 0.
+__device__ __forceinline__ uint32_t inv(uint32_t o)
 {
-  v = (v >> 1) ^ static_cast<uint32_t>(static_cast<int32_t>(v << 31) >> 31);
-  if (v & 0xff000000u) {
-    if (v >= 0x80000000u) v += 0x01000000u;
-    v += 0x80000000u;
-  }
-  return (v << 31) | (v >> 1);
+  const uint32_t r = __funnelshift_r(o, o, 1);
+  const uint32_t even = static_cast<int32_t>(r) >= 0x01000000 ? r + 0x80000000u : r;
+  const uint32_t v = static_cast<int32_t>(r) < 0 ? 0x00ffffffu - r : even;
+  return __funnelshift_r(v, v, 1);
 }
 
-__device__ __forceinline__ uint64_t inv(uint64_t v)
+__device__ __forceinline__ uint64_t inv(uint64_t o)
 {
-  const uint32_t h = static_cast<uint32_t>(v >> 32);
-  const uint32_t l = static_cast<uint32_t>(v);
-  const uint32_t sg = 0u - (l & 1u);                       // (v << 63) >> 63 arithmetic
-  uint32_t nh = (h >> 1) ^ sg;
-  const uint32_t nl = __funnelshift_r(l, h, 1) ^ sg;
-  if (nh & 0xffe00000u) {
-    if (nh >= 0x80000000u) nh += 0x00200000u;
-    nh += 0x80000000u;
-  }
-  const uint32_t oh = __funnelshift_r(nh, nl, 1);          // rotate right by 1
-  const uint32_t ol = __funnelshift_r(nl, nh, 1);
-  return (static_cast<uint64_t>(oh) << 32) | ol;
+  const uint32_t h = static_cast<uint32_t>(o >> 32);
+  const uint32_t l = static_cast<uint32_t>(o);
+  const uint32_t rh = __funnelshift_r(h, l, 1);
+  const uint32_t rl = __funnelshift_r(l, h, 1);
+  const uint32_t even = static_cast<int32_t>(rh) >= 0x00200000 ? rh + 0x80000000u : rh;
+  const bool odd = static_cast<int32_t>(rh) < 0;
+  const uint32_t vh = odd ? 0x001fffffu - rh : even;
+  const uint32_t vl = odd ? ~rl : rl;
+  const uint32_t xh = __funnelshift_r(vh, vl, 1);
+  const uint32_t xl = __funnelshift_r(vl, vh, 1);
+  return (static_cast<uint64_t>(xh) << 32) | xl;
 }
 
 __device__ __forceinline__ uint32_t quant(uint32_t val, const QParams& q)
@@ -514,16 +499,60 @@ __device__ __forceinline__ uint64_t dequant_fp(uint64_t enc, const QParams& q)
   return dec | (enc << 63);
 }
 
-// dequant_fp of a 64-bit code below 2^32 (a chunk whose widths are all at most
-// 32): a = ceil(enc / 2) < 2^31 never reaches the 2^52 escape, and the u32 ->
-// f64 conversion is exact, so the result equals dequant_fp's.
-__device__ __forceinline__ uint64_t dequant_fp_narrow(uint32_t enc, const QParams& q)
+// The same for codes that cannot be escapes, as every code of a narrow subchunk: with
+// z the code's zigzag integer (enc / 2, or -(enc + 1) / 2 for odd codes; its magnitude
+// is a above and its sign the value's), the value is z * 2^(thr_e - bias - m), both
+// factors and the product exact.  32-bit codes below 2^23, 64-bit ones below 2^32.
+__device__ __forceinline__ uint32_t dequant_plain32(uint32_t enc, const QParams& q)
 {
-  if (enc == 0u) return 0ull;
-  const uint32_t a = (enc >> 1) + (enc & 1u);
+  const int z = static_cast<int>((enc >> 1) ^ (0u - (enc & 1u)));
+  const float scale = __uint_as_float(static_cast<uint32_t>(q.thr_e - 23) << 23);
+  return __float_as_uint(__fmul_rn(__int2float_rn(z), scale));
+}
+
+__device__ __forceinline__ uint64_t dequant_plain64(uint32_t enc, const QParams& q)
+{
+  const int z = static_cast<int>((enc >> 1) ^ (0u - (enc & 1u)));
   const double scale = __longlong_as_double(static_cast<long long>(q.thr_e - 52) << 52);
-  const uint64_t dec = static_cast<uint64_t>(__double_as_longlong(__dmul_rn(__uint2double_rn(a), scale)));
-  return dec | (static_cast<uint64_t>(enc & 1u) << 63);
+  return static_cast<uint64_t>(__double_as_longlong(__dmul_rn(__int2double_rn(z), scale)));
+}
+
+// Quantize for ordinary values, as nearly all are: |v| below quant_limit, which
+// excludes escapes, NaN and infinities (and every value where eb_e = 0, whose integer
+// form differs), and for 64-bit values keeps the code below 2^31.  floor(y + 1/2) as
+// one fused multiply-add rounded down and a truncation (see above); then 2 enc - sign,
+// but 0 for enc = 0.  The 64-bit limit is a high word, compared as a float: words that
+// are no number as a float are large.
+__device__ __forceinline__ float quant_limit32(const QParams& q)
+{
+  return q.eb_e ? __uint_as_float(static_cast<uint32_t>(q.thr_e) << 23) : 0.0f;
+}
+__device__ __forceinline__ float quant_limit64(const QParams& q)
+{
+  return q.eb_e ? __uint_as_float(static_cast<uint32_t>(q.thr_e - 23) << 20) : 0.0f;
+}
+__device__ __forceinline__ bool quant_ordinary(uint32_t word, float limit)  // a value, or a 64-bit value's high word
+{
+  return fabsf(__uint_as_float(word)) < limit;
+}
+__device__ __forceinline__ uint32_t quant_plain(uint32_t v, float inv_scale)
+{
+  const uint32_t e = __float2uint_rz(__fmaf_rd(fabsf(__uint_as_float(v)), inv_scale, 0.5f));
+  return static_cast<uint32_t>(max(static_cast<int>(2u * e - (v >> 31)), 0));
+}
+__device__ __forceinline__ uint32_t quant_plain(uint32_t l, uint32_t h, double inv_scale)
+{
+  const double v = fabs(__hiloint2double(static_cast<int>(h), static_cast<int>(l)));
+  const uint32_t e = __double2uint_rz(__fma_rd(v, inv_scale, 0.5));
+  return static_cast<uint32_t>(max(static_cast<int>(2u * e - (h >> 31)), 0));
+}
+__device__ __forceinline__ float quant_scale32(const QParams& q)  // 2^(150 - thr_e)
+{
+  return __uint_as_float(static_cast<uint32_t>(277 - q.thr_e) << 23);
+}
+__device__ __forceinline__ double quant_scale64(const QParams& q)  // 2^(1075 - thr_e)
+{
+  return __longlong_as_double(static_cast<long long>(2098 - q.thr_e) << 52);
 }
 
 template <bool LOSSY, typename T>
@@ -540,104 +569,11 @@ __device__ __forceinline__ T decode_value(T v, const QParams& q)
   else return inv(v);
 }
 
-__device__ __forceinline__ int bit_width(uint32_t m) { return m ? 32 - __clz(m) : 0; }
-__device__ __forceinline__ int bit_width(uint64_t m) { return m ? 64 - __clzll(m) : 0; }
-
-__device__ __forceinline__ uint32_t warp_max(uint32_t v) { return __reduce_max_sync(0xffffffffu, v); }
-__device__ __forceinline__ uint64_t warp_max(uint64_t v)
-{
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const uint64_t w = __shfl_xor_sync(0xffffffffu, v, o);
-    v = w > v ? w : v;
-  }
-  return v;
-}
-
-// bit width of the largest value held by the warp, from the OR of all values
-__device__ __forceinline__ int warp_bit_width(uint32_t v)
-{
-  return bit_width(__reduce_or_sync(0xffffffffu, v));
-}
-__device__ __forceinline__ int warp_bit_width(uint64_t v)
-{
-  const uint32_t hi = __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(v >> 32));
-  const uint32_t lo = __reduce_or_sync(0xffffffffu, static_cast<uint32_t>(v));
-  return hi ? 64 - __clz(hi) : bit_width(lo);
-}
-
 __device__ __forceinline__ long long warp_sum(long long v)
 {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
-}
-
-// ----------------------------------------------------------------------------
-// Decoupled look-back over flag words.  Called by one whole warp for item
-// `idx` whose segment starts at `seg_begin` (items before the segment count as
-// an inclusive prefix of 0).  Each poll reads the 32 nearest unresolved flags
-// (one load per lane), sums the run of aggregates up to the
-// nearest inclusive prefix, and slides past runs of aggregates; it only waits
-// when the nearest unresolved flag is not published yet.  Returns the exclusive
-// prefix, or -1 when a wait exceeded `limit_ns` or another CTA already
-// reported an error in the counter block `hdr`.
-// ----------------------------------------------------------------------------
-__device__ __forceinline__ long long lookback(const uint64_t* flags, long long idx, long long seg_begin,
-                                              const uint64_t* hdr, unsigned long long limit_ns = SPIN_TIMEOUT_NS)
-{
-  constexpr int PER = 1;  // polls of 32 flags: measured against 64 and 128, encode +2 % and +4-9 %
-  const int lane = threadIdx.x & 31;
-  long long excl = 0;
-  long long end = idx - 1;
-  unsigned long long t0 = 0;
-  unsigned sleep_ns = 256;
-  int polls = 0;
-  while (true) {
-    uint64_t f[PER];
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const long long j = end - lane - 32 * k;
-      f[k] = (j >= seg_begin) ? ld_relaxed_u64(&flags[j]) : FLAG_INC;
-    }
-    int z = 32 * PER;  // distance of the nearest unpublished flag
-    int p = 32 * PER;  // distance of the nearest inclusive prefix
-#pragma unroll
-    for (int k = PER - 1; k >= 0; --k) {
-      const unsigned nr = __ballot_sync(0xffffffffu, (f[k] >> 62) == 0ull);
-      const unsigned inc = __ballot_sync(0xffffffffu, (f[k] >> 62) == 2ull);
-      if (nr) z = 32 * k + __ffs(nr) - 1;
-      if (inc) p = 32 * k + __ffs(inc) - 1;
-    }
-    if (p < z) {
-      long long s = 0;
-#pragma unroll
-      for (int k = 0; k < PER; ++k)
-        if (lane + 32 * k <= p) s += static_cast<long long>(f[k] & FLAG_VAL);
-      return excl + warp_sum(s);
-    }
-    if (z > 0) {
-      long long s = 0;
-#pragma unroll
-      for (int k = 0; k < PER; ++k)
-        if (lane + 32 * k < z) s += static_cast<long long>(f[k] & FLAG_VAL);
-      excl += warp_sum(s);
-      end -= z;
-      continue;
-    }
-    // the nearest predecessor has not published yet: back off, bounded in time
-    if (++polls == 64) {
-      t0 = globaltimer_ns();
-    } else if (polls > 64 && (polls & 63) == 0) {
-      const bool late = globaltimer_ns() - t0 > limit_ns;
-      const bool failed = ld_relaxed_u64(&hdr[WS_STATUS]) != 0ull;
-      if (__any_sync(0xffffffffu, late || failed)) return -1;
-    }
-    // sleeping from the first miss keeps hundreds of waiting warps from flooding
-    // the L2 with polls (measured: decode +3-8 %, encode unchanged)
-    __nanosleep(sleep_ns);
-    if (sleep_ns < 2048) sleep_ns <<= 1;
-  }
 }
 
 // ----------------------------------------------------------------------------
@@ -741,7 +677,8 @@ struct ChunkScan {
   // One warp: the sum of the sizes of all chunks before `idx`, or -1 when a wait
   // exceeded the limit or another CTA reported an error in the counter block.
   // Where `from` lies in the own group, only of chunks [from, idx).
-  __device__ long long prefix(long long idx, long long from, const uint64_t* hdr) const
+  __device__ long long prefix(long long idx, long long from, const uint64_t* hdr,
+                              unsigned long long limit_ns = SPIN_TIMEOUT_NS) const
   {
     const int lane = threadIdx.x & 31;
     const long long own = idx / GROUP;
@@ -781,7 +718,7 @@ struct ChunkScan {
       if (++polls == 256) {
         t0 = globaltimer_ns();
       } else if (polls > 256 && (polls & 255) == 0) {
-        const bool late = globaltimer_ns() - t0 > SPIN_TIMEOUT_NS;
+        const bool late = globaltimer_ns() - t0 > limit_ns;
         const bool failed = ld_relaxed_u64(&hdr[WS_STATUS]) != 0ull;
         if (__any_sync(0xffffffffu, late || failed)) return -1;
       }
@@ -886,36 +823,6 @@ __device__ __forceinline__ void store_shifted(uint8_t* dst, const uint8_t* src, 
       if (r >= 0 && r < len) a0[16 * e + (tid & 15)] = src[r];
     }
   }
-}
-
-// Reads the u32 word starting at an arbitrary byte offset of 16-byte aligned
-// shared memory (the two aligned words around it, funnel-shifted).
-__device__ __forceinline__ uint32_t lds_u32_at_byte(const uint8_t* base, int byte_off)
-{
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(base);
-  const int wi = byte_off >> 2;
-  const int sh = (byte_off & 3) * 8;
-  return __funnelshift_r(w[wi], w[wi + 1], sh);
-}
-
-// Extracts `ln` bits (1 <= ln <= 64) starting at bit `pos` of 16-byte aligned
-// shared memory, LSB-first little-endian (the stream's bit order).
-__device__ __forceinline__ uint32_t extract_bits32(const uint32_t* w, int pos, int ln)
-{
-  const int wi = pos >> 5;
-  const uint32_t v = __funnelshift_r(w[wi], w[wi + 1], pos & 31);
-  return ln >= 32 ? v : (v & ((1u << ln) - 1u));
-}
-
-__device__ __forceinline__ uint64_t extract_bits64(const uint32_t* w, int pos, int ln)
-{
-  const int wi = pos >> 5;
-  const int sh = pos & 31;
-  const uint32_t w0 = w[wi], w1 = w[wi + 1], w2 = w[wi + 2];
-  const uint32_t lo = __funnelshift_r(w0, w1, sh);
-  const uint32_t hi = __funnelshift_r(w1, w2, sh);
-  const uint64_t v = (static_cast<uint64_t>(hi) << 32) | lo;
-  return ln >= 64 ? v : (v & ((1ull << ln) - 1ull));
 }
 
 // ----------------------------------------------------------------------------

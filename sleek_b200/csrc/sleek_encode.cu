@@ -38,29 +38,19 @@ constexpr int EW_STAGE = EW_IN + CS;    // room before them for the packed chunk
 constexpr int EW_G = 4;  // subchunks whose loads, maps and reductions overlap
 
 // Quantizes one group's values (EW_G subchunks, this lane's 16 bytes of each) when
-// all of the warp's are ordinary: |v| small enough that the code needs at most 30
-// bits (f64) or is not an escape (f32).  False (nothing written) otherwise.
+// all of the warp's are ordinary (see quant_plain).  False (nothing written) otherwise.
 __device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], uint32_t (&o)[EW_G], float limit, float inv_scale)
 {
   bool odd = false;
 #pragma unroll
-  for (int u = 0; u < EW_G; ++u) {
-    odd |= !(fabsf(__uint_as_float(w[u].x)) < limit);
-    odd |= !(fabsf(__uint_as_float(w[u].y)) < limit);
-    odd |= !(fabsf(__uint_as_float(w[u].z)) < limit);
-    odd |= !(fabsf(__uint_as_float(w[u].w)) < limit);
-  }
+  for (int u = 0; u < EW_G; ++u)
+    odd |= !quant_ordinary(w[u].x, limit) | !quant_ordinary(w[u].y, limit) | !quant_ordinary(w[u].z, limit) |
+           !quant_ordinary(w[u].w, limit);
   if (__any_sync(0xffffffffu, odd)) return false;
-  auto one = [&](uint32_t v) {
-    const uint32_t e = __float2uint_rz(__fmaf_rd(fabsf(__uint_as_float(v)), inv_scale, 0.5f));
-    return static_cast<uint32_t>(max(static_cast<int>(2u * e - (v >> 31)), 0));
-  };
 #pragma unroll
   for (int u = 0; u < EW_G; ++u) {
-    w[u].x = one(w[u].x);
-    w[u].y = one(w[u].y);
-    w[u].z = one(w[u].z);
-    w[u].w = one(w[u].w);
+    w[u] = make_uint4(quant_plain(w[u].x, inv_scale), quant_plain(w[u].y, inv_scale), quant_plain(w[u].z, inv_scale),
+                      quant_plain(w[u].w, inv_scale));
     o[u] = w[u].x | w[u].y | w[u].z | w[u].w;
   }
   return true;
@@ -70,23 +60,11 @@ __device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], uint32_t (&o)[EW_G
 {
   bool odd = false;
 #pragma unroll
-  for (int u = 0; u < EW_G; ++u) {
-    // the high words, ordered like floats (those that are no number as a float are large)
-    odd |= !(fabsf(__uint_as_float(w[u].y)) < limit);
-    odd |= !(fabsf(__uint_as_float(w[u].w)) < limit);
-  }
+  for (int u = 0; u < EW_G; ++u) odd |= !quant_ordinary(w[u].y, limit) | !quant_ordinary(w[u].w, limit);
   if (__any_sync(0xffffffffu, odd)) return false;
-  auto one = [&](uint32_t l, uint32_t h) {
-    const double v = fabs(__hiloint2double(static_cast<int>(h), static_cast<int>(l)));
-    const uint32_t e = __double2uint_rz(__fma_rd(v, inv_scale, 0.5));
-    return static_cast<uint32_t>(max(static_cast<int>(2u * e - (h >> 31)), 0));
-  };
 #pragma unroll
   for (int u = 0; u < EW_G; ++u) {
-    w[u].x = one(w[u].x, w[u].y);
-    w[u].z = one(w[u].z, w[u].w);
-    w[u].y = 0u;
-    w[u].w = 0u;
+    w[u] = make_uint4(quant_plain(w[u].x, w[u].y, inv_scale), 0u, quant_plain(w[u].z, w[u].w, inv_scale), 0u);
     o[u] = w[u].x | w[u].z;
   }
   return true;
@@ -101,16 +79,15 @@ __device__ __forceinline__ int encode_values(uint8_t* data, const QParams& q, in
   using T = EncVal<KIND>;
   constexpr bool LOSSY = (KIND & 2) != 0;
   uint32_t hi_or = 0, lo_or = 0;  // OR of the codes of subchunk `lane`
-  // ordinary values of the quantizer (see quant_group)
   float limit = 0.0f;
   typename std::conditional<sizeof(T) == 4, float, double>::type inv_scale = 0;
   if constexpr (LOSSY) {
     if constexpr (sizeof(T) == 4) {
-      limit = q.eb_e ? __uint_as_float(static_cast<uint32_t>(q.thr_e) << 23) : 0.0f;
-      inv_scale = __uint_as_float(static_cast<uint32_t>(277 - q.thr_e) << 23);
+      limit = quant_limit32(q);
+      inv_scale = quant_scale32(q);
     } else {
-      limit = q.eb_e ? __uint_as_float(static_cast<uint32_t>(q.thr_e - 23) << 20) : 0.0f;
-      inv_scale = __longlong_as_double(static_cast<long long>(2098 - q.thr_e) << 52);
+      limit = quant_limit64(q);
+      inv_scale = quant_scale64(q);
     }
   }
 #pragma unroll 1
@@ -614,7 +591,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB)
       if (excl >= 0) {
         uint64_t* const start = a.starts + job;
         if (k.c == 0) {
-          if (lane == 0) st_relaxed_u64(start, FLAG_INC | static_cast<uint64_t>(excl));
+          if (lane == 0) st_relaxed_u64(start, FLAG_SET | static_cast<uint64_t>(excl));
           excl = 0;
         } else if (seg < k.g / GROUP * GROUP) {
           const uint64_t v = ChunkScan::await(start, hdr);

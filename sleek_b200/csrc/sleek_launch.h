@@ -1,5 +1,5 @@
 // sleek_launch.h -- host-side launch interface between the C ABI (sleek_capi.cu)
-// and the kernels (sleek_kernels.cu).  Internal to the library.
+// and the kernels (sleek_decode.cu).  Internal to the library.
 #pragma once
 
 #include <cstdint>
@@ -8,8 +8,6 @@
 struct sleek_stream_info;
 
 namespace sleek {
-
-constexpr int NT_MAX_WARPS = 32;
 
 // lossy quantizer parameters, as sleek_error_bound derives them
 // (include/sleek_lossy_gpu.h:47-71 of the reference)
@@ -68,13 +66,12 @@ struct BatchDecArgs {
   const long long* chunk_base;  // device: first chunk id of each job by capacity, then the total
   int njobs;
   uint64_t* ws;                 // zeroed workspace header words
-  long long* offsets;           // workspace: payload offset of every chunk id
-  long long* actual;            // workspace: chunks in each stream (from its header)
-  long long* actual_insize;     // workspace: bytes each stream decodes to
+  unsigned long long* places;   // workspace: of every chunk id its offset in the stream | size << 48
+  long long* actual;            // workspace: bytes each stream decodes to
 };
 
 // Launch shapes of the single-buffer kernels (sleek_encode.cu: EncShape*,
-// sleek_kernels.cu: DecShape*); shape 0 is the default.  Every shape produces the same bytes.
+// sleek_decode.cu: DecShape*); shape 0 is the default.  Every shape produces the same bytes.
 struct ShapeInfo {
   int threads;        // per CTA
   int warps;          // warps that work on chunks
@@ -82,6 +79,8 @@ struct ShapeInfo {
   int ctas_per_sm;    // CTAs per SM the registers are budgeted for
 };
 int shape_count(bool enc);
+// the shape that stands for shape 0 where no other was asked for, by the number of chunks
+int default_shape(bool enc, long long chunks, int sms);
 ShapeInfo shape_info(bool enc, int shape);
 cudaError_t launch_encode(int width, bool lossy, int shape, const EncArgs& a, int grid, cudaStream_t st);
 cudaError_t launch_decode(int width, bool lossy, int shape, const DecArgs& a, int grid, cudaStream_t st);

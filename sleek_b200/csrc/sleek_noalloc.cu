@@ -13,7 +13,7 @@
 // output.
 //
 // The scratch holds the same things the regular entry point's workspace holds (a
-// header of 32 words and one look-back flag per 16 KB chunk), so its fixed size
+// header of 32 words and one word per 16 KB chunk), so its fixed size
 // bounds the input: at most SLEEK_STATIC_MAX_INPUT_BYTES (1 GiB) per call.
 #include <cstdint>
 #include <mutex>

@@ -1,8 +1,8 @@
 // sleek_selftest.cu -- device self-tests of the codec's building blocks.
 //
 // Bounded waits: without faulting or hanging the device, one CTA waits on an
-// mbarrier that nothing arrives on, and one warp looks back over a predecessor
-// flag that nothing publishes, each with a caller-given limit, using the same
+// mbarrier that nothing arrives on, and one warp waits for the size of a preceding
+// chunk that nothing publishes, each with a caller-given limit, using the same
 // wait helpers as the encode and decode kernels (sleek_device.cuh).  Both must
 // give up, report it, and return; the context stays usable.
 //
@@ -21,11 +21,12 @@
 namespace sleek {
 namespace {
 
-// result[0]: 1 if the mbarrier wait gave up; result[1]: the look-back's return
+// result[0]: 1 if the mbarrier wait gave up; result[1]: the prefix's return
 // value (-1 when it gave up); result[2]: nanoseconds the two waits took
 __global__ void __launch_bounds__(32) k_selftest_waits(unsigned long long limit_ns, uint64_t* flags, long long* result)
 {
   __shared__ __align__(8) uint64_t bar;
+  __shared__ ScanRing ring;
   const int lane = threadIdx.x;
   if (lane == 0) {
     mbar_init(&bar, 1);  // expects one arrival, which never comes
@@ -34,9 +35,9 @@ __global__ void __launch_bounds__(32) k_selftest_waits(unsigned long long limit_
   __syncwarp();
   const unsigned long long t0 = globaltimer_ns();
   const bool got = mbar_wait_bounded(&bar, 0, limit_ns);
-  // flags[0] is the unpublished predecessor of item 1; flags[2..] hold the
-  // workspace header the look-back reads for errors (status word 0: none)
-  const long long lb = lookback(flags + 2 + WS_HDR_WORDS, 1, 0, flags + 2, limit_ns);
+  // the size of chunk 0 is never published; flags[2..] hold the workspace header
+  // that the wait reads for errors (status word 0: none)
+  const long long lb = ChunkScan(flags + 2 + WS_HDR_WORDS, 2, &ring).prefix(1, 0, flags + 2, limit_ns);
   const unsigned long long t1 = globaltimer_ns();
   if (lane == 0) {
     result[0] = got ? 0 : 1;
@@ -173,11 +174,14 @@ __global__ void __launch_bounds__(256) k_selftest_maps(unsigned long long n, uns
     } else if constexpr (CHECK == 1) {  // f32 quantize, every word x 8 bounds
       const uint32_t v = static_cast<uint32_t>(i);
       const QParams q = q32(static_cast<int>(i >> 32));
-      ok = quant_fp(v, q) == lit_quant<uint32_t>(v, q.eb_e, q.thr_e, static_cast<uint32_t>(q.offs));
+      const uint32_t want = lit_quant<uint32_t>(v, q.eb_e, q.thr_e, static_cast<uint32_t>(q.offs));
+      ok = quant_fp(v, q) == want &&
+           (!quant_ordinary(v, quant_limit32(q)) || quant_plain(v, quant_scale32(q)) == want);
     } else if constexpr (CHECK == 2) {  // f32 dequantize, every code x 8 bounds
       const uint32_t e = static_cast<uint32_t>(i);
       const QParams q = q32(static_cast<int>(i >> 32));
-      ok = dequant_fp(e, q) == lit_dequant<uint32_t>(e, q.thr_e, static_cast<uint32_t>(q.offs));
+      const uint32_t want = lit_dequant<uint32_t>(e, q.thr_e, static_cast<uint32_t>(q.offs));
+      ok = dequant_fp(e, q) == want && (e >= (1u << 23) || dequant_plain32(e, q) == want);
     } else if constexpr (CHECK == 3) {  // f64 forward transform and inverse, every sign/exponent x 2^20
       const uint64_t v = word64(i >> 20, i & 0xfffff);
       const uint64_t t = fwd(v);
@@ -186,14 +190,16 @@ __global__ void __launch_bounds__(256) k_selftest_maps(unsigned long long n, uns
       const uint64_t v = word64((i >> 20) & 0xfff, i & 0xfffff);
       const QParams q = q64(static_cast<int>(i >> 32));
       const uint64_t want = lit_quant<uint64_t>(v, q.eb_e, q.thr_e, q.offs);
-      ok = quant_fp(v, q) == want && quant(v, q) == want;
-    } else {  // f64 dequantize x 9 bounds: every code below 2^32 (also the narrow
+      const uint32_t h = static_cast<uint32_t>(v >> 32);
+      ok = quant_fp(v, q) == want && quant(v, q) == want &&
+           (!quant_ordinary(h, quant_limit64(q)) || quant_plain(static_cast<uint32_t>(v), h, quant_scale64(q)) == want);
+    } else {  // f64 dequantize x 9 bounds: every code below 2^32 (also the plain
               // form), then codes of every bit length
       const QParams q = q64(static_cast<int>((i >> 32) % 9));
       if ((i >> 32) < 9) {
         const uint32_t e = static_cast<uint32_t>(i);
         const uint64_t want = lit_dequant<uint64_t>(e, q.thr_e, q.offs);
-        ok = dequant_fp(static_cast<uint64_t>(e), q) == want && dequant_fp_narrow(e, q) == want &&
+        ok = dequant_fp(static_cast<uint64_t>(e), q) == want && dequant_plain64(e, q) == want &&
              dequant(static_cast<uint64_t>(e), q) == want;
       } else {
         const int len = static_cast<int>((i >> 26) & 63) + 1;
