@@ -258,6 +258,11 @@ __global__ void __launch_bounds__(NTEAM * TW * 32, MINB) k_decode(const DecArgs 
   const int warp = tid >> 5;
   const int team = warp / TW;
   const int cw = warp % TW;
+  if (tid == 0) {
+    for (int i = 0; i < 2 * NTEAM; ++i) mbar_init(&bars[i], 1);
+    mbar_fence_init();
+  }
+  grid_wait();
   const WsPhase ph = WsPhase::of(a.ws, a.flag_cap);  // self-resetting workspace
   uint64_t* const hdr = ph.hdr;
   const uint16_t* const size_in = reinterpret_cast<const uint16_t*>(a.in + 8);
@@ -302,10 +307,6 @@ __global__ void __launch_bounds__(NTEAM * TW * 32, MINB) k_decode(const DecArgs 
   const long long g_chunks = a.out_cap > 0 ? (a.out_cap + CS - 1) / CS : -1;
   const bool spec = g_chunks > 0 && a.in_len >= 8 + 2 * g_chunks;
   const long long insize = *reinterpret_cast<const long long*>(a.in);
-  if (tid == 0) {
-    for (int i = 0; i < 2 * NTEAM; ++i) mbar_init(&bars[i], 1);
-    mbar_fence_init();
-  }
   if (spec) sum_groups(0, min(g_chunks, static_cast<long long>(DEC_WINDOW)));
 
   // header checks (every CTA reads the 8-byte header)
@@ -463,6 +464,7 @@ __global__ void __launch_bounds__(NTEAM * TW * 32, MINB) k_decode(const DecArgs 
   if (warp == NW - 1) ph.clear_other_share(lane);
 
   // ---- epilogue ------------------------------------------------------------------
+  grid_release();
   __syncthreads();
   if (tid == 0) {
     __threadfence();
@@ -494,6 +496,8 @@ __global__ void __launch_bounds__(PRE_NT) k_decode_prepass(const BatchDecArgs a)
 {
   __shared__ uint32_t wsum[PRE_NT / 32];
   __shared__ int wbad[PRE_NT / 32];
+  grid_release();
+  grid_wait();
   const int j = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const BatchJob& job = a.jobs[j];
@@ -560,11 +564,12 @@ __global__ void __launch_bounds__(DB_NT, 1) k_decode_batch(const BatchDecArgs a)
   const int team = warp / DB_TW, cw = warp % DB_TW;
   const bool leads = lane == 0 && cw == 0;
   uint64_t* const ws = a.ws;
-  for (int i = tid; i <= a.njobs; i += DB_NT) cb[i] = a.chunk_base[i];
   if (tid == 0) {
     for (int i = 0; i < DB_TEAMS; ++i) mbar_init(&bars[i], 1);
     mbar_fence_init();
   }
+  grid_wait();
+  for (int i = tid; i <= a.njobs; i += DB_NT) cb[i] = a.chunk_base[i];
   __syncthreads();
   const long long total = cb[a.njobs];
   const bool failed_before = ld_relaxed_u64(&ws[WS_STATUS]) != 0ull;  // the prepass found an error
@@ -654,6 +659,7 @@ __global__ void __launch_bounds__(DB_NT, 1) k_decode_batch(const BatchDecArgs a)
   }
 
   // ---- epilogue: an error anywhere turns every size into -status ---------------
+  grid_release();
   __syncthreads();
   __shared__ int last_cta;
   if (tid == 0) {
@@ -699,8 +705,7 @@ static cudaError_t launch_dec_k(const DecArgs& a, int grid, cudaStream_t st)
   static unsigned long long attr = 0;
   cudaError_t e = ensure_smem_attr(k, S::SMEM, &attr);
   if (e != cudaSuccess) return e;
-  k<<<grid, S::NT, S::SMEM, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(k, grid, S::NT, S::SMEM, st, a);
 }
 
 template <typename T, bool LOSSY, class S>
@@ -771,14 +776,12 @@ int default_shape(bool enc, long long chunks, int sms)
 
 cudaError_t launch_decode_batch(const BatchDecArgs& a, int grid, cudaStream_t st)
 {
-  k_decode_prepass<<<a.njobs, PRE_NT, 0, st>>>(a);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_after(k_decode_prepass, a.njobs, PRE_NT, 0, st, a);
   if (e != cudaSuccess) return e;
   static unsigned long long attr = 0;
   e = ensure_smem_attr(k_decode_batch, DB_SMEM, &attr);
   if (e != cudaSuccess) return e;
-  k_decode_batch<<<grid, DB_NT, DB_SMEM, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(k_decode_batch, grid, DB_NT, DB_SMEM, st, a);
 }
 
 int decode_batch_blocks_per_sm()

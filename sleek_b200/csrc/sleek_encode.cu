@@ -457,6 +457,11 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB)
   uint8_t* const stg = smem + warp * EW_STAGE;
   uint64_t* const bar = bars + warp;
 
+  if (tid == 0) {
+    for (int i = 0; i < NW; ++i) mbar_init(&bars[i], 1);
+    mbar_fence_init();
+  }
+  grid_wait();
   const WsPhase ph = [&]() {
     if constexpr (BATCH) return WsPhase::fixed(a.ws);
     else return WsPhase::of(a.ws, a.flag_cap);
@@ -478,8 +483,6 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB)
   const int first_n = static_cast<int>(share < NW ? share : NW);
   if (tid == 0) {
     s_first = atomicAdd(tick, static_cast<unsigned long long>(first_n));
-    for (int i = 0; i < NW; ++i) mbar_init(&bars[i], 1);
-    mbar_fence_init();
     ring.known = 0;
     ring.gone = 0;
   }
@@ -630,6 +633,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB)
   }
 
   // ---- epilogue: the last CTA out finishes the outputs -----------------------
+  grid_release();
   __syncthreads();
   __shared__ int last_cta;
   if (tid == 0) {
@@ -690,8 +694,7 @@ static cudaError_t launch_enc_k(const EncArgs& a, int grid, cudaStream_t st)
   static unsigned long long attr = 0;
   cudaError_t e = ensure_smem_attr(k, S::SMEM, &attr);
   if (e != cudaSuccess) return e;
-  k<<<grid, S::NT, S::SMEM, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(k, grid, S::NT, S::SMEM, st, a);
 }
 
 template <int KIND, class S>
@@ -760,8 +763,7 @@ cudaError_t launch_encode_batch(const BatchEncArgs& a, int grid, cudaStream_t st
   static unsigned long long attr = 0;
   cudaError_t e = ensure_smem_attr(k, ENC_BATCH_SMEM, &attr);
   if (e != cudaSuccess) return e;
-  k<<<grid, EncShapeBatch::NT, ENC_BATCH_SMEM, st>>>(a);
-  return cudaGetLastError();
+  return launch_after(k, grid, EncShapeBatch::NT, ENC_BATCH_SMEM, st, a);
 }
 
 int encode_batch_blocks_per_sm()
