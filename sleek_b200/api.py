@@ -13,6 +13,7 @@ Calls are asynchronous on the current torch CUDA stream unless ``check=True``.
 from __future__ import annotations
 
 import ctypes as C
+from functools import lru_cache
 from typing import NamedTuple, Optional
 
 import numpy as np
@@ -33,14 +34,23 @@ class ErrorBoundInfo(NamedTuple):
     dtype: np.dtype
 
     def c_struct(self):
-        if self.dtype == np.float32:
-            return _capi.EbInfoF32(self.eb_e, self.thr_e, self.offs_e)
-        return _capi.EbInfoF64(self.eb_e, self.thr_e, self.offs_e)
+        return _c_struct(self.eb_e, self.thr_e, self.offs_e, np.dtype(self.dtype).itemsize)
+
+
+@lru_cache(maxsize=256)
+def _c_struct(eb_e, thr_e, offs_e, itemsize):
+    return (_capi.EbInfoF32 if itemsize == 4 else _capi.EbInfoF64)(eb_e, thr_e, offs_e)
 
 
 def sleek_upper_bound_size(insize: int) -> int:
     """Bytes to allocate for the stream of an insize-byte input (sleek_common_gpu.h:79-83)."""
     return int(_capi.lib().sleek_upper_bound_size(int(insize)))
+
+
+def _upper_bound(insize: int) -> int:
+    """sleek_upper_bound_size of a size that is not negative, without the call."""
+    chunks = (insize + CS - 1) // CS
+    return 12 + chunks * (CS + 2)
 
 
 def sleek_system_checks() -> int:
@@ -72,18 +82,26 @@ def sleek_error_bound(eb, dtype=None) -> ErrorBoundInfo:
     return ErrorBoundInfo(info.eb_e, info.thr_e, info.offs_e, dtype)
 
 
+_NP_DTYPES = {torch.float32: np.dtype(np.float32), torch.float64: np.dtype(np.float64)}
+
+
 def _np_dtype(t: torch.Tensor) -> np.dtype:
-    if t.dtype == torch.float32:
-        return np.dtype(np.float32)
-    if t.dtype == torch.float64:
-        return np.dtype(np.float64)
-    raise TypeError("SLEEK compresses float32 and float64 data")
+    dt = _NP_DTYPES.get(t.dtype)
+    if dt is None:
+        raise TypeError("SLEEK compresses float32 and float64 data")
+    return dt
 
 
 def _stream_handle(stream) -> int:
-    if stream is None:
-        stream = torch.cuda.current_stream()
+    if stream is None:  # the current device's current stream, without a Stream object
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     return int(stream.cuda_stream) if isinstance(stream, torch.cuda.Stream) else int(stream)
+
+
+@lru_cache(maxsize=None)
+def _entry(name: str, lossy: bool, itemsize: int):
+    """The C ABI's compress or decompress function of one kind."""
+    return getattr(_capi.lib(), f"sleek_{name}{'_lossy' if lossy else ''}_f{8 * itemsize}")
 
 
 def _ws(workspace):
@@ -120,25 +138,25 @@ def sleek_compress_gpu(blocks: int, *args, stream=None, workspace=None, check: b
     d_input, num_elements, d_encoded, d_encsize = args
     _check_device(d_input, d_encoded, d_encsize)
     dt = _np_dtype(d_input)
+    w = dt.itemsize
+    n = int(num_elements)
     if num_elements > d_input.numel():
         raise SleekError(_capi.SLEEK_ERR_INVALID_ARG, "sleek_compress_gpu: num_elements exceeds the input")
-    if d_encoded.numel() * d_encoded.element_size() < sleek_upper_bound_size(num_elements * dt.itemsize):
+    if d_encoded.numel() * d_encoded.element_size() < _upper_bound(n * w):
         raise SleekError(_capi.SLEEK_ERR_CAPACITY, "sleek_compress_gpu: d_encoded smaller than the upper bound")
     if d_encsize.dtype != torch.int64:
         raise TypeError("d_encsize must be an int64 tensor")
-    L = _capi.lib()
     wp, wb = _ws(workspace)
     st = _stream_handle(stream)
-    t = "f32" if dt == np.float32 else "f64"
     if eb_info is None:
-        rc = getattr(L, f"sleek_compress_{t}")(d_input.data_ptr(), int(num_elements), d_encoded.data_ptr(),
-                                               d_encsize.data_ptr(), wp, wb, st)
+        rc = _entry("compress", False, w)(d_input.data_ptr(), n, d_encoded.data_ptr(), d_encsize.data_ptr(), wp, wb, st)
     else:
         if eb_info.dtype != dt:
             raise TypeError("eb_info dtype does not match the input dtype")
-        rc = getattr(L, f"sleek_compress_lossy_{t}")(eb_info.c_struct(), d_input.data_ptr(), int(num_elements),
-                                                     d_encoded.data_ptr(), d_encsize.data_ptr(), wp, wb, st)
-    _capi.check(rc, "sleek_compress_gpu")
+        rc = _entry("compress", True, w)(eb_info.c_struct(), d_input.data_ptr(), n, d_encoded.data_ptr(),
+                                         d_encsize.data_ptr(), wp, wb, st)
+    if rc:
+        _capi.check(rc, "sleek_compress_gpu")
     if check:
         _raise_if_negative(d_encsize, "sleek_compress_gpu")
 
@@ -162,20 +180,20 @@ def sleek_decompress_gpu(blocks: int, *args, stream=None, workspace=None, check:
         raise TypeError("d_decsize must be an int64 tensor")
     if encoded_bytes is None or encoded_bytes < 0:
         encoded_bytes = -1
-    cap = d_decoded.numel() * d_decoded.element_size()
-    L = _capi.lib()
+    w = dt.itemsize
+    cap = d_decoded.numel() * w
     wp, wb = _ws(workspace)
     st = _stream_handle(stream)
-    t = "f32" if dt == np.float32 else "f64"
     if eb_info is None:
-        rc = getattr(L, f"sleek_decompress_{t}")(d_encoded.data_ptr(), int(encoded_bytes), d_decoded.data_ptr(),
-                                                 cap, d_decsize.data_ptr(), wp, wb, st)
+        rc = _entry("decompress", False, w)(d_encoded.data_ptr(), int(encoded_bytes), d_decoded.data_ptr(), cap,
+                                            d_decsize.data_ptr(), wp, wb, st)
     else:
         if eb_info.dtype != dt:
             raise TypeError("eb_info dtype does not match the output dtype")
-        rc = getattr(L, f"sleek_decompress_lossy_{t}")(eb_info.c_struct(), d_encoded.data_ptr(), int(encoded_bytes),
-                                                       d_decoded.data_ptr(), cap, d_decsize.data_ptr(), wp, wb, st)
-    _capi.check(rc, "sleek_decompress_gpu")
+        rc = _entry("decompress", True, w)(eb_info.c_struct(), d_encoded.data_ptr(), int(encoded_bytes),
+                                           d_decoded.data_ptr(), cap, d_decsize.data_ptr(), wp, wb, st)
+    if rc:
+        _capi.check(rc, "sleek_decompress_gpu")
     if check:
         _raise_if_negative(d_decsize, "sleek_decompress_gpu")
 
