@@ -695,7 +695,7 @@ struct DecShape {
 // with 4 teams of two, which do not cover the latencies).
 using DecShape0 = DecShape<6, 2, 1>;  // default
 using DecShape1 = DecShape<10, 1, 1>;
-using DecShape2 = DecShape<1, 8, 3>;
+using DecShape2 = DecShape<2, 8, 2>;
 constexpr int DEC_SHAPES = 3;
 
 template <typename T, bool LOSSY, class S>
@@ -764,14 +764,13 @@ ShapeInfo shape_info(bool enc, int shape)
 
 int shape_count(bool enc) { return enc ? encode_shape_count() : DEC_SHAPES; }
 
-// Decode with at most one chunk per resident CTA of shape 2: eight warps share each
-// chunk, so its decode takes a quarter of the time (f32, lossless / eb 1e-3: 4 KB
-// 4.8 / 4.7 us against 7.2 / 6.5 with shape 0; 2.4 MB 6.1 / 6.3 against 6.9 / 7.5;
-// 4.8 MB 7.0 / 7.0 against 7.7 / 7.5).  Beyond that its CTAs' second round costs more
-// than it gains (19 MB: 12.8 / 13.1 against 12.7 / 11.2).
+// Decode with at most one chunk per SM: shape 2, whose eight warps share a chunk (f32
+// lossless, microseconds on the GPU against shape 0's: 200 KB 6.0 / 6.5, 1.6 MB 6.1 /
+// 6.4; with more chunks its larger CTAs cost more than they gain: 3 MB 7.6 / 6.1).
 int default_shape(bool enc, long long chunks, int sms)
 {
-  return !enc && chunks <= static_cast<long long>(DecShape2::MINB) * sms ? 2 : 0;
+  if (enc) return encode_default_shape(chunks, sms);
+  return chunks <= sms ? 2 : 0;
 }
 
 cudaError_t launch_decode_batch(const BatchDecArgs& a, int grid, cudaStream_t st)

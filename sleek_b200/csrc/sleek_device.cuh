@@ -184,6 +184,11 @@ __device__ __forceinline__ void st_relaxed_u64(uint64_t* p, uint64_t v)
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+__device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v)
+{
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ uint64_t ld_relaxed_u64(const uint64_t* p)
 {
   uint64_t v;
@@ -627,7 +632,7 @@ struct ChunkScan {
   // one thread: the size of chunk `idx` is known
   __device__ void publish(long long idx, uint32_t csize) const
   {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(flags + idx), "r"(csize) : "memory");
+    st_relaxed_u32(flags + idx, csize);
     if (chunks > GROUP)
       asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(sums + idx / GROUP), "l"((1ull << 32) | csize)
                    : "memory");
@@ -735,6 +740,34 @@ struct ChunkScan {
       }
       __nanosleep(64);
     }
+  }
+
+  // One warp: the same from the flags alone, for a few groups, with no scanner.
+  __device__ long long prefix_flags(long long idx, const uint64_t* hdr) const
+  {
+    const int lane = threadIdx.x & 31;
+    long long excl = 0;
+    unsigned long long t0 = 0;
+    int polls = 0;
+    for (long long b = 0; b < idx; b += GROUP) {
+      while (true) {
+        uint32_t s;
+        const bool ok = part(b, idx < b + GROUP ? idx : b + GROUP, lane, &s);
+        if (__all_sync(0xffffffffu, ok)) {
+          excl += __reduce_add_sync(0xffffffffu, s);
+          break;
+        }
+        if (++polls == 256) {
+          t0 = globaltimer_ns();
+        } else if (polls > 256 && (polls & 255) == 0) {
+          const bool late = globaltimer_ns() - t0 > SPIN_TIMEOUT_NS;
+          const bool failed = ld_relaxed_u64(&hdr[WS_STATUS]) != 0ull;
+          if (__any_sync(0xffffffffu, late || failed)) return -1;
+        }
+        __nanosleep(32);
+      }
+    }
+    return excl;
   }
 
   // One warp: the value another warp puts at `p` (never 0), or 0 when the wait gave up.

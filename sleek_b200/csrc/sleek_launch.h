@@ -86,6 +86,7 @@ cudaError_t launch_encode(int width, bool lossy, int shape, const EncArgs& a, in
 cudaError_t launch_decode(int width, bool lossy, int shape, const DecArgs& a, int grid, cudaStream_t st);
 int blocks_per_sm(int width, bool lossy, bool enc, int shape);
 int encode_shape_count();
+int encode_default_shape(long long chunks, int sms);
 ShapeInfo encode_shape_info(int shape);
 int encode_blocks_per_sm(int width, bool lossy, int shape);
 cudaError_t launch_decode_batch(const BatchDecArgs& a, int grid, cudaStream_t st);

@@ -1,13 +1,14 @@
 """The encoder's packing and placing at the widths, alignments and chunk mixes where
 its paths change: every code width (whole and joined runs), chunks stored raw among
 compressed ones (places at other alignments than expected), inputs at every element
-offset, and more than two groups of 64 chunks, alone and in a batch."""
+offset, and more than two groups of 64 chunks, alone (one warp per chunk, and the
+several warps per chunk of small inputs) and in a batch."""
 import numpy as np
 import pytest
 import torch
 
 from oracle import oracle as O
-from sleek_b200 import api
+from sleek_b200 import _capi, api
 from sleek_b200.batch import compress_batch
 
 pytestmark = pytest.mark.gpu
@@ -40,14 +41,31 @@ def _codes(dt, case, seed):
 CASES = ["each width", "mixed widths", "around a word", "raw among packed"]
 
 
+@pytest.fixture
+def default_shapes():
+    yield
+    for w in (4, 8):
+        for lossy in (0, 1):
+            _capi.check(_capi.lib().sleek_set_launch_shape(0, w, lossy, -1, 0, 0))
+
+
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 @pytest.mark.parametrize("case", CASES)
 @pytest.mark.parametrize("eb", [None, 0.5])
-def test_widths_and_places(cuda, dt, case, eb):
+def test_widths_and_places(cuda, default_shapes, dt, case, eb):
     x = _codes(dt, case, 5)[:-3]
-    for first in range(16 // x.itemsize):
-        t = torch.from_numpy(np.concatenate([np.zeros(first, dt), x])).cuda()[first:]
-        assert api.compress(t, eb).cpu().numpy().tobytes() == O.encode(x, eb), first
+    want = O.encode(x, eb)
+    for ctas in (0, 1):  # by the number of chunks; one warp per chunk for any number
+        _capi.check(_capi.lib().sleek_set_launch_shape(0, x.itemsize, int(eb is not None), -1, 0, ctas))
+        for first in range(16 // x.itemsize):
+            t = torch.from_numpy(np.concatenate([np.zeros(first, dt), x])).cuda()[first:]
+            assert api.compress(t, eb).cpu().numpy().tobytes() == want, (ctas, first)
+
+
+@pytest.mark.parametrize("chunks", [1, 2, 591, 592, 593])
+def test_sizes_around_the_small_inputs(cuda, chunks):
+    x = np.resize(_codes(np.float32, "mixed widths", 7), chunks * 4096 - 1)
+    assert api.compress(torch.from_numpy(x).cuda(), 0.5).cpu().numpy().tobytes() == O.encode(x, 0.5)
 
 
 def test_batch_places_over_groups(cuda):
