@@ -39,7 +39,7 @@ constexpr int EW_G = 4;  // subchunks whose loads, maps and reductions overlap
 
 // Quantizes one group's values (EW_G subchunks, this lane's 16 bytes of each) when
 // all of the warp's are ordinary (see quant_plain).  False (nothing written) otherwise.
-__device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], uint32_t (&o)[EW_G], float limit, float inv_scale)
+__device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], float limit, float inv_scale)
 {
   bool odd = false;
 #pragma unroll
@@ -51,12 +51,11 @@ __device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], uint32_t (&o)[EW_G
   for (int u = 0; u < EW_G; ++u) {
     w[u] = make_uint4(quant_plain(w[u].x, inv_scale), quant_plain(w[u].y, inv_scale), quant_plain(w[u].z, inv_scale),
                       quant_plain(w[u].w, inv_scale));
-    o[u] = w[u].x | w[u].y | w[u].z | w[u].w;
   }
   return true;
 }
 
-__device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], uint32_t (&o)[EW_G], float limit, double inv_scale)
+__device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], float limit, double inv_scale)
 {
   bool odd = false;
 #pragma unroll
@@ -65,58 +64,76 @@ __device__ __forceinline__ bool quant_group(uint4 (&w)[EW_G], uint32_t (&o)[EW_G
 #pragma unroll
   for (int u = 0; u < EW_G; ++u) {
     w[u] = make_uint4(quant_plain(w[u].x, w[u].y, inv_scale), 0u, quant_plain(w[u].z, w[u].w, inv_scale), 0u);
-    o[u] = w[u].x | w[u].z;
   }
   return true;
 }
 
+// This lane's 16 bytes of values to codes, whatever the values are.
+template <int KIND>
+__device__ __forceinline__ uint4 encode_any(const uint4 w, const QParams& q)
+{
+  constexpr bool LOSSY = (KIND & 2) != 0;
+  if constexpr ((KIND & 1) == 0) {
+    return make_uint4(encode_value<LOSSY>(w.x, q), encode_value<LOSSY>(w.y, q), encode_value<LOSSY>(w.z, q),
+                      encode_value<LOSSY>(w.w, q));
+  } else {
+    const uint64_t a = encode_value<LOSSY>((static_cast<uint64_t>(w.y) << 32) | w.x, q);
+    const uint64_t b = encode_value<LOSSY>((static_cast<uint64_t>(w.w) << 32) | w.z, q);
+    return make_uint4(static_cast<uint32_t>(a), static_cast<uint32_t>(a >> 32), static_cast<uint32_t>(b),
+                      static_cast<uint32_t>(b >> 32));
+  }
+}
+
 // One warp: values to codes for the EW_G subchunks from i0 on (this lane's 16 bytes of
-// each to `w`, and back to the stage if KEEP); returns the bit width of subchunk `lane`
-// where it is one of them, else 0.
-template <int KIND, bool KEEP>
+// each to `w`, and if STAGED back to the stage); returns the bit width of subchunk
+// `lane` where it is one of them, else 0.  SMALL (and STAGED) keeps the code small: a
+// group with values that are not ordinary goes subchunk by subchunk through a loop.
+template <int KIND, bool STAGED, bool SMALL>
 __device__ __forceinline__ int encode_group(uint8_t* data, uint4 (&w)[EW_G], int i0, const QParams& q, int lane)
 {
-  using T = EncVal<KIND>;
   constexpr bool LOSSY = (KIND & 2) != 0;
+  constexpr bool WIDE = (KIND & 1) != 0;
   uint32_t hi_or = 0, lo_or = 0;  // OR of the codes of subchunk `lane`
-  uint32_t o[EW_G];
   uint4* const p = reinterpret_cast<uint4*>(data + i0 * 512 + lane * 16);
 #pragma unroll
   for (int u = 0; u < EW_G; ++u) w[u] = p[32 * u];
-  bool done = false;
+  bool done = false;  // (then 64-bit codes are below 2^31)
   if constexpr (LOSSY) {
-    if constexpr (sizeof(T) == 4) done = quant_group(w, o, quant_limit32(q), quant_scale32(q));
-    else done = quant_group(w, o, quant_limit64(q), quant_scale64(q));
+    if constexpr (WIDE) done = quant_group(w, quant_limit64(q), quant_scale64(q));
+    else done = quant_group(w, quant_limit32(q), quant_scale32(q));
+    if (SMALL && !done) {
+#pragma unroll 1
+      for (int u = 0; u < EW_G; ++u) {
+        const uint4 v = encode_any<KIND>(p[32 * u], q);
+        p[32 * u] = v;
+        const uint32_t r = __reduce_or_sync(0xffffffffu, WIDE ? v.x | v.z : v.x | v.y | v.z | v.w);
+        if (lane == i0 + u) lo_or = r;
+        if (WIDE) {
+          const uint32_t h = __reduce_or_sync(0xffffffffu, v.y | v.w);
+          if (lane == i0 + u) hi_or = h;
+        }
+      }
+      return hi_or ? 64 - __clz(hi_or) : 32 - __clz(lo_or);
+    }
+    if (!done) {
+#pragma unroll
+      for (int u = 0; u < EW_G; ++u) w[u] = encode_any<KIND>(w[u], q);
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < EW_G; ++u) w[u] = encode_any<KIND>(w[u], q);
   }
-  if (!done) {
-    uint32_t oh[EW_G];
+  if (WIDE && !done) {
 #pragma unroll
     for (int u = 0; u < EW_G; ++u) {
-      if constexpr (sizeof(T) == 4) {
-        w[u] = make_uint4(encode_value<LOSSY>(w[u].x, q), encode_value<LOSSY>(w[u].y, q),
-                          encode_value<LOSSY>(w[u].z, q), encode_value<LOSSY>(w[u].w, q));
-        o[u] = w[u].x | w[u].y | w[u].z | w[u].w;
-      } else {
-        const uint64_t a = encode_value<LOSSY>((static_cast<uint64_t>(w[u].y) << 32) | w[u].x, q);
-        const uint64_t b = encode_value<LOSSY>((static_cast<uint64_t>(w[u].w) << 32) | w[u].z, q);
-        w[u] = make_uint4(static_cast<uint32_t>(a), static_cast<uint32_t>(a >> 32), static_cast<uint32_t>(b),
-                          static_cast<uint32_t>(b >> 32));
-        o[u] = w[u].x | w[u].z;
-        oh[u] = w[u].y | w[u].w;
-      }
-    }
-    if constexpr (sizeof(T) == 8) {
-#pragma unroll
-      for (int u = 0; u < EW_G; ++u) {
-        const uint32_t r = __reduce_or_sync(0xffffffffu, oh[u]);
-        if (lane == i0 + u) hi_or = r;
-      }
+      const uint32_t r = __reduce_or_sync(0xffffffffu, w[u].y | w[u].w);
+      if (lane == i0 + u) hi_or = r;
     }
   }
 #pragma unroll
   for (int u = 0; u < EW_G; ++u) {
-    if (KEEP) p[32 * u] = w[u];
-    const uint32_t r = __reduce_or_sync(0xffffffffu, o[u]);
+    if (STAGED) p[32 * u] = w[u];
+    const uint32_t r = __reduce_or_sync(0xffffffffu, WIDE ? w[u].x | w[u].z : w[u].x | w[u].y | w[u].z | w[u].w);
     if (lane == i0 + u) lo_or = r;
   }
   return hi_or ? 64 - __clz(hi_or) : 32 - __clz(lo_or);
@@ -125,14 +142,19 @@ __device__ __forceinline__ int encode_group(uint8_t* data, uint4 (&w)[EW_G], int
 // One warp: the staged chunk's values become codes in place (each lane reads and
 // writes its own 16 bytes of every subchunk); returns the bit width of subchunk
 // `lane`.
-template <int KIND>
+//
+// SMALL: a batch's warps work on four kinds at once, whose code does not fit the
+// instruction cache beside each other; smaller code took a batch of 60 arrays from
+// 73.1 to 69.0 us (and the loop below unrolled, which takes 2 % off one kind's
+// calls, from 73 to 84 and 105 by twos and fours).
+template <int KIND, bool SMALL>
 __device__ __forceinline__ int encode_values(uint8_t* data, const QParams& q, int lane)
 {
   int ln = 0;
-#pragma unroll 1
+#pragma unroll (SMALL ? 1 : 4)
   for (int i0 = 0; i0 < SC; i0 += EW_G) {
     uint4 w[EW_G];
-    ln += encode_group<KIND, true>(data, w, i0, q, lane);
+    ln += encode_group<KIND, true, SMALL>(data, w, i0, q, lane);
   }
   return ln;
 }
@@ -255,6 +277,13 @@ struct Packer {
       else put_short(b * (m * m) + a, 4 * ln);
     }
   }
+  // 8 <= ln <= 15
+  __device__ __forceinline__ void mid32(const uint4 w, int ln)
+  {
+    const uint32_t m = 1u << ln;
+    const uint32_t a = w.y * m + w.x, b = w.w * m + w.z;
+    put<32, 64>(b * (m * m) + a, __funnelshift_l(b, 0u, 2 * ln), 0u, 0u, 4 * ln);
+  }
   // 4 <= ln <= 15
   __device__ __forceinline__ void narrow32(const uint4 w, int ln)
   {
@@ -304,7 +333,7 @@ struct Packer {
 // bytes, the packed bits, the int16 trailer.  In place, subchunk by subchunk: the
 // packed bytes of a subchunk end before the codes of the next one begin, and a
 // lane's stores follow an exchange that every lane enters with its codes loaded.
-template <typename T>
+template <typename T, bool SMALL>
 __device__ __forceinline__ void pack_chunk(uint8_t* stg, int a, int ln, int osize, int lane)
 {
   constexpr int B = static_cast<int>(sizeof(T));
@@ -317,15 +346,16 @@ __device__ __forceinline__ void pack_chunk(uint8_t* stg, int a, int ln, int osiz
   const uint32_t l2 = __shfl_sync(0xffffffffu, ln, 30) | (__shfl_sync(0xffffffffu, ln, 31) << 8);
   k.carry = k.half ? l2 : 0u;
   const unsigned wide = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 16 && ln < 32) : (ln >= 32 && ln < 64));
-  const unsigned narrow = B == 8 ? __ballot_sync(0xffffffffu, ln >= 16 && ln < 32) : 0u;
+  const unsigned narrow = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 8 && ln < 16) : (ln >= 16 && ln < 32));
   const unsigned any = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 4 && ln < 16) : (ln >= 8 && ln < 32));
 #pragma unroll 1
   for (int i0 = 0; i0 < SC; i0 += EW_G) {
+    const uint4* const in = reinterpret_cast<const uint4*>(stg + EW_IN + i0 * 512 + lane * 16);
     uint4 w[EW_G];
     int l[EW_G];
 #pragma unroll
     for (int u = 0; u < EW_G; ++u) {
-      w[u] = *reinterpret_cast<const uint4*>(stg + EW_IN + (i0 + u) * 512 + lane * 16);
+      w[u] = in[32 * u];
       l[u] = __shfl_sync(0xffffffffu, ln, i0 + u);
     }
     constexpr unsigned ALL = (1u << EW_G) - 1u;
@@ -335,20 +365,30 @@ __device__ __forceinline__ void pack_chunk(uint8_t* stg, int a, int ln, int osiz
         if constexpr (B == 4) k.wide32(w[u], l[u]);
         else k.wide64(w[u], l[u]);
       }
-    } else if (B == 8 && ((narrow >> i0) & ALL) == ALL) {
+    } else if (((narrow >> i0) & ALL) == ALL) {
 #pragma unroll
-      for (int u = 0; u < EW_G; ++u) k.narrow64(w[u], l[u]);
+      for (int u = 0; u < EW_G; ++u) {
+        if constexpr (B == 4) k.mid32(w[u], l[u]);
+        else k.narrow64(w[u], l[u]);
+      }
     } else if (((any >> i0) & ALL) == ALL) {
 #pragma unroll
       for (int u = 0; u < EW_G; ++u) {
         if constexpr (B == 4) k.narrow32(w[u], l[u]);
         else k.any64(w[u], l[u]);
       }
-    } else {
+    } else if constexpr (!SMALL) {
 #pragma unroll
       for (int u = 0; u < EW_G; ++u) {
         if constexpr (B == 4) k.put32(w[u], l[u]);
         else k.put64(w[u], l[u]);
+      }
+    } else {
+#pragma unroll 1
+      for (int u = 0; u < EW_G; ++u) {
+        const int l1 = __shfl_sync(0xffffffffu, ln, i0 + u);
+        if constexpr (B == 4) k.put32(in[32 * u], l1);
+        else k.put64(in[32 * u], l1);
       }
     }
   }
@@ -540,13 +580,13 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB)
     }
     int ln;
     if constexpr (KIND >= 0) {
-      ln = encode_values<KIND>(stg + EW_IN, k.q, lane);
+      ln = encode_values<KIND, false>(stg + EW_IN, k.q, lane);
     } else {
       switch (k.kind) {
-        case 0: ln = encode_values<0>(stg + EW_IN, k.q, lane); break;
-        case 1: ln = encode_values<1>(stg + EW_IN, k.q, lane); break;
-        case 2: ln = encode_values<2>(stg + EW_IN, k.q, lane); break;
-        default: ln = encode_values<3>(stg + EW_IN, k.q, lane); break;
+        case 0: ln = encode_values<0, true>(stg + EW_IN, k.q, lane); break;
+        case 1: ln = encode_values<1, true>(stg + EW_IN, k.q, lane); break;
+        case 2: ln = encode_values<2, true>(stg + EW_IN, k.q, lane); break;
+        default: ln = encode_values<3, true>(stg + EW_IN, k.q, lane); break;
       }
     }
     const bool wide = (KIND >= 0 ? KIND : k.kind) & 1;
@@ -570,8 +610,8 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB)
       long long guess = 2 * k.c;
       if constexpr (!BATCH) guess = scan.guess(k.g);
       al = static_cast<int>((reinterpret_cast<uintptr_t>(k.out) + 8 + 2 * k.chunks + guess) & 15u);
-      if (wide) pack_chunk<uint64_t>(stg, al, ln, k.osize, lane);
-      else pack_chunk<uint32_t>(stg, al, ln, k.osize, lane);
+      if (wide) pack_chunk<uint64_t, BATCH>(stg, al, ln, k.osize, lane);
+      else pack_chunk<uint32_t, BATCH>(stg, al, ln, k.osize, lane);
       fence_proxy_async_smem();
       __syncwarp();
     }
@@ -728,7 +768,7 @@ __global__ void __launch_bounds__(ENC_TEAM * 32, ENC_TEAM_CTAS) k_encode_team(co
     const bool wlate = __any_sync(0xffffffffu, late);
     uint4 w[EW_G];
     int width = 0;
-    if (!wlate) width = encode_group<KIND, false>(stg, w, warp * EW_G, a.q, lane);
+    if (!wlate) width = encode_group<KIND, false, false>(stg, w, warp * EW_G, a.q, lane);
     if (lane / EW_G == warp) s_ln[lane] = width;
     if (__syncthreads_or(wlate)) {
       if (tid == 0) set_status(ph.hdr, ST_TIMEOUT, c);
