@@ -89,24 +89,26 @@ __device__ __forceinline__ uint4 codes_narrow(const uint32_t* w, int bit, int ln
   }
 }
 template <int B>
-__device__ __forceinline__ uint4 codes_wide(const uint32_t* w, int bit, int ln, int lane)  // 16 .. 31 / 32 .. 63
+__device__ __forceinline__ uint4 codes_wide(const uint32_t* w, int bit, int ln, int lane)  // 16 .. 32 / 32 .. 64
 {
   const int at = bit + lane * ((16 / B) * ln);
   const uint32_t* const p = w + (at >> 5);
   const uint32_t w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = p[4];
   const uint32_t x0 = __funnelshift_r(w0, w1, at), x1 = __funnelshift_r(w1, w2, at);
   const uint32_t x2 = __funnelshift_r(w2, w3, at), x3 = __funnelshift_r(w3, w4, at);
+  // (shifts of up to 32: the clamping form)
   if constexpr (B == 4) {
-    const uint32_t m = (1u << ln) - 1u;
+    const uint32_t m = pow2_or_0(ln) - 1u;
     const bool far = 3 * ln >= 64;
-    return make_uint4(x0 & m, __funnelshift_r(x0, x1, ln) & m, __funnelshift_r(x1, x2, 2 * ln) & m,
-                      __funnelshift_r(far ? x2 : x1, far ? x3 : x2, 3 * ln) & m);
+    return make_uint4(x0 & m, __funnelshift_rc(x0, x1, ln) & m, __funnelshift_rc(x1, x2, 2 * ln - 32) & m,
+                      __funnelshift_rc(far ? x2 : x1, far ? x3 : x2, 3 * ln - (far ? 64 : 32)) & m);
   } else {
-    const uint32_t m = (1u << (ln - 32)) - 1u;
-    return make_uint4(x0, x1 & m, __funnelshift_r(x1, x2, ln), __funnelshift_r(x2, x3, ln) & m);
+    const int k = ln - 32;
+    const uint32_t m = pow2_or_0(k) - 1u;
+    return make_uint4(x0, x1 & m, __funnelshift_rc(x1, x2, k), __funnelshift_rc(x2, x3, k) & m);
   }
 }
-// codes as wide as the values, or 16 raw bytes at any bit offset
+// 16 raw bytes at any bit offset
 __device__ __forceinline__ uint4 codes_full(const uint32_t* w, int bit, int lane)
 {
   const int at = bit + lane * 128;
@@ -151,7 +153,7 @@ __device__ __forceinline__ bool decode_chunk(const uint8_t* stg, int sft, int cs
   // widths of the narrow form, of the wide one, and (32-bit values) without escapes
   constexpr int NARROW = B == 4 ? 16 : 32;
   const unsigned narrow = __ballot_sync(0xffffffffu, ln < NARROW);
-  const unsigned wide = __ballot_sync(0xffffffffu, ln >= NARROW && ln < 2 * NARROW);
+  const unsigned wide = __ballot_sync(0xffffffffu, ln >= NARROW);
   const unsigned plain = B == 4 && LOSSY ? __ballot_sync(0xffffffffu, ln < 24) : narrow;
   auto unpack = [&](auto full) {
     auto put = [&](int i, const uint4 v) {
@@ -189,8 +191,7 @@ __device__ __forceinline__ bool decode_chunk(const uint8_t* stg, int sft, int cs
 #pragma unroll
         for (int u = 0; u < DEC_G; ++u) {
           if (l[u] < NARROW) e[u] = codes_narrow<B>(w, b[u], l[u], lane);
-          else if (l[u] < 2 * NARROW) e[u] = codes_wide<B>(w, b[u], l[u], lane);
-          else e[u] = codes_full(w, b[u], lane);
+          else e[u] = codes_wide<B>(w, b[u], l[u], lane);
         }
 #pragma unroll
         for (int u = 0; u < DEC_G; ++u) {

@@ -571,6 +571,14 @@ __device__ __forceinline__ double quant_scale64(const QParams& q)  // 2^(1075 - 
   return __longlong_as_double(static_cast<long long>(2098 - q.thr_e) << 52);
 }
 
+// 2^n for n < 32, and 0 for n = 32
+__device__ __forceinline__ uint32_t pow2_or_0(int n)
+{
+  uint32_t r;
+  asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(n));
+  return r;
+}
+
 template <bool LOSSY, typename T>
 __device__ __forceinline__ T encode_value(T v, const QParams& q)
 {

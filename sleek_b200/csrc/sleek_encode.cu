@@ -266,9 +266,7 @@ struct Packer {
   __device__ __forceinline__ void put32(const uint4 w, int ln)
   {
     if (ln == 0) return;
-    if (ln == 32) {
-      put<64, 128>(w.x, w.y, w.z, w.w, 128);
-    } else if (ln >= 16) {
+    if (ln >= 16) {
       wide32(w, ln);
     } else {
       const uint32_t m = 1u << ln;
@@ -291,30 +289,29 @@ struct Packer {
     const uint32_t a = w.y * m + w.x, b = w.w * m + w.z;
     put_any(b * (m * m) + a, __funnelshift_l(b, 0u, 2 * ln), 4 * ln);
   }
-  // 16 <= ln <= 31
+  // 16 <= ln <= 32 (shifts of up to 32: the clamping form)
   __device__ __forceinline__ void wide32(const uint4 w, int ln)
   {
-    const uint32_t m = 1u << ln;
-    const uint32_t a0 = w.y * m + w.x, a1 = __funnelshift_l(w.y, 0u, ln);
-    const uint32_t b0 = w.w * m + w.z, b1 = __funnelshift_l(w.w, 0u, ln);
+    const uint32_t m = pow2_or_0(ln);
+    const uint32_t a0 = w.y * m + w.x, a1 = __funnelshift_lc(w.y, 0u, ln);
+    const uint32_t b0 = w.w * m + w.z, b1 = __funnelshift_lc(w.w, 0u, ln);
     const int k = 2 * ln - 32;
-    put<64, 128>(a0, b0 * (1u << k) + a1, __funnelshift_l(b0, b1, k), __funnelshift_l(b1, 0u, k), 4 * ln);
+    put<64, 128>(a0, b0 * pow2_or_0(k) + a1, __funnelshift_lc(b0, b1, k), __funnelshift_lc(b1, 0u, k), 4 * ln);
   }
 
   // one subchunk of 64-bit codes, this lane's two
   __device__ __forceinline__ void put64(const uint4 w, int ln)
   {
     if (ln == 0) return;
-    if (ln == 64) put<64, 128>(w.x, w.y, w.z, w.w, 128);
-    else if (ln >= 32) wide64(w, ln);
+    if (ln >= 32) wide64(w, ln);
     else if (ln >= 16) narrow64(w, ln);
     else put_short(w.z * (1u << ln) + w.x, 2 * ln);
   }
-  // 32 <= ln <= 63
+  // 32 <= ln <= 64
   __device__ __forceinline__ void wide64(const uint4 w, int ln)
   {
     const int k = ln - 32;
-    put<64, 128>(w.x, w.z * (1u << k) + w.y, __funnelshift_l(w.z, w.w, k), __funnelshift_l(w.w, 0u, k), 2 * ln);
+    put<64, 128>(w.x, w.z * pow2_or_0(k) + w.y, __funnelshift_lc(w.z, w.w, k), __funnelshift_lc(w.w, 0u, k), 2 * ln);
   }
   // 16 <= ln <= 31
   __device__ __forceinline__ void narrow64(const uint4 w, int ln)
@@ -345,7 +342,7 @@ __device__ __forceinline__ void pack_chunk(uint8_t* stg, int a, int ln, int osiz
   // the last two widths share the first word with the packed bits
   const uint32_t l2 = __shfl_sync(0xffffffffu, ln, 30) | (__shfl_sync(0xffffffffu, ln, 31) << 8);
   k.carry = k.half ? l2 : 0u;
-  const unsigned wide = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 16 && ln < 32) : (ln >= 32 && ln < 64));
+  const unsigned wide = __ballot_sync(0xffffffffu, ln >= (B == 4 ? 16 : 32));
   const unsigned narrow = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 8 && ln < 16) : (ln >= 16 && ln < 32));
   const unsigned any = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 4 && ln < 16) : (ln >= 8 && ln < 32));
 #pragma unroll 1
