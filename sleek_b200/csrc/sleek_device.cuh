@@ -536,8 +536,8 @@ __device__ __forceinline__ uint64_t dequant_plain64(uint32_t enc, const QParams&
 // Quantize for ordinary values, as nearly all are: |v| below quant_limit, which
 // excludes escapes, NaN and infinities (and every value where eb_e = 0, whose integer
 // form differs), and for 64-bit values keeps the code below 2^31.  floor(y + 1/2) as
-// one fused multiply-add rounded down and a truncation (see above); then 2 enc - sign,
-// but 0 for enc = 0.  The 64-bit limit is a high word, compared as a float: words that
+// one fused multiply-add rounded down and its integer part (see above); then
+// 2 enc - sign, but 0 for enc = 0.  The 64-bit limit is a high word, compared as a float: words that
 // are no number as a float are large.
 __device__ __forceinline__ float quant_limit32(const QParams& q)
 {
@@ -553,8 +553,13 @@ __device__ __forceinline__ bool quant_ordinary(uint32_t word, float limit)  // a
 }
 __device__ __forceinline__ uint32_t quant_plain(uint32_t v, float inv_scale)
 {
-  const uint32_t e = __float2uint_rz(__fmaf_rd(fabsf(__uint_as_float(v)), inv_scale, 0.5f));
-  return static_cast<uint32_t>(max(static_cast<int>(2u * e - (v >> 31)), 0));
+  // t <= 2^23, so 2^23 + t rounded down is 2^23 + floor(t), whose bits are those of
+  // 2^23 plus floor(t): no conversion, of which an SM does 16 a cycle (40 MB f32 slab
+  // 34.1 -> 33.4 us, batch of 60 arrays 68.1 -> 67.2)
+  const float t = __fmaf_rd(fabsf(__uint_as_float(v)), inv_scale, 0.5f);
+  const uint32_t e = __float_as_uint(__fadd_rd(t, 8388608.0f));  // + 0x4b000000
+  const uint32_t c = 0x6a000000u + static_cast<uint32_t>(static_cast<int32_t>(v) >> 31);  // -2 * 0x4b000000 - sign
+  return static_cast<uint32_t>(max(static_cast<int>(2u * e + c), 0));
 }
 __device__ __forceinline__ uint32_t quant_plain(uint32_t l, uint32_t h, double inv_scale)
 {
@@ -571,7 +576,7 @@ __device__ __forceinline__ double quant_scale64(const QParams& q)  // 2^(1075 - 
   return __longlong_as_double(static_cast<long long>(2098 - q.thr_e) << 52);
 }
 
-// 2^n for n < 32, and 0 for n = 32
+// 2^n for n < 32, 0 for larger n
 __device__ __forceinline__ uint32_t pow2_or_0(int n)
 {
   uint32_t r;

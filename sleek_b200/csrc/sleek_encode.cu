@@ -186,8 +186,7 @@ struct Packer {
     if constexpr (MAXR > 64) {
       y3 = __funnelshift_l(x2, x3, s);
       const uint32_t y4 = __funnelshift_l(x3, 0u, s);
-      tail = t < 96 ? y2 : (t < 128 ? y3 : y4);
-      if (MINR < 64 && t < 64) tail = y1;
+      tail = MINR < 64 && t < 64 ? y1 : (t < 96 ? y2 : (t < 128 ? y3 : y4));
     } else {
       tail = t < 64 ? y1 : y2;
     }
@@ -299,6 +298,17 @@ struct Packer {
     put<64, 128>(a0, b0 * pow2_or_0(k) + a1, __funnelshift_lc(b0, b1, k), __funnelshift_lc(b1, 0u, k), 4 * ln);
   }
 
+  // 8 <= ln <= 32, without a branch: the products and shifts that do not apply are 0
+  __device__ __forceinline__ void long32(const uint4 w, int ln)
+  {
+    const uint32_t m = pow2_or_0(ln);
+    const uint32_t a0 = w.y * m + w.x, a1 = __funnelshift_lc(w.y, 0u, ln);
+    const uint32_t b0 = w.w * m + w.z, b1 = __funnelshift_lc(w.w, 0u, ln);
+    const int k = max(2 * ln - 32, 0);
+    const uint32_t x1 = 2 * ln < 32 ? __funnelshift_l(b0, 0u, 2 * ln) : b0 * pow2_or_0(k) + a1;
+    put<32, 128>(b0 * pow2_or_0(2 * ln) + a0, x1, __funnelshift_lc(b0, b1, k), __funnelshift_lc(b1, 0u, k), 4 * ln);
+  }
+
   // one subchunk of 64-bit codes, this lane's two
   __device__ __forceinline__ void put64(const uint4 w, int ln)
   {
@@ -344,6 +354,7 @@ __device__ __forceinline__ void pack_chunk(uint8_t* stg, int a, int ln, int osiz
   k.carry = k.half ? l2 : 0u;
   const unsigned wide = __ballot_sync(0xffffffffu, ln >= (B == 4 ? 16 : 32));
   const unsigned narrow = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 8 && ln < 16) : (ln >= 16 && ln < 32));
+  const unsigned lng = B == 4 ? __ballot_sync(0xffffffffu, ln >= 8) : 0u;
   const unsigned any = __ballot_sync(0xffffffffu, B == 4 ? (ln >= 4 && ln < 16) : (ln >= 8 && ln < 32));
 #pragma unroll 1
   for (int i0 = 0; i0 < SC; i0 += EW_G) {
@@ -368,6 +379,9 @@ __device__ __forceinline__ void pack_chunk(uint8_t* stg, int a, int ln, int osiz
         if constexpr (B == 4) k.mid32(w[u], l[u]);
         else k.narrow64(w[u], l[u]);
       }
+    } else if (B == 4 && ((lng >> i0) & ALL) == ALL) {
+#pragma unroll
+      for (int u = 0; u < EW_G; ++u) k.long32(w[u], l[u]);
     } else if (((any >> i0) & ALL) == ALL) {
 #pragma unroll
       for (int u = 0; u < EW_G; ++u) {
