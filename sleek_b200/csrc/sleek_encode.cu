@@ -539,6 +539,35 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB)
   const ChunkScan scan(ph.flags, total, &ring);
 
   uint32_t par = 0;
+  auto job_of = [&](long long g) {  // last job whose first chunk id is <= g (empty jobs are skipped)
+    int lo = 0;
+    if constexpr (BATCH) {
+      int hi = a.njobs - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (cb[mid] <= g) lo = mid;
+        else hi = mid - 1;
+      }
+    }
+    return lo;
+  };
+  // the 16 KB, 16-byte aligned, that hold nearly all of chunk g if it is a whole one
+  auto whole_chunk = [&](long long g) -> const uint8_t* {
+    const uint8_t* in;
+    long long c = g, insize;
+    if constexpr (BATCH) {
+      const int lo = job_of(g);
+      c = g - cb[lo];
+      in = a.jobs[lo].in;
+      insize = a.jobs[lo].insize;
+    } else {
+      in = a.in;
+      insize = a.insize;
+    }
+    if ((c + 1) * CS > insize) return nullptr;
+    in += c * CS;
+    return in - (reinterpret_cast<uintptr_t>(in) & 15u);
+  };
   auto next = [&]() -> long long {
     unsigned long long t = 0;
     if (lane == 0) t = atomicAdd(tick, 1ull);
@@ -554,12 +583,7 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB)
     long long seg = 0;
     int job = 0;
     if constexpr (BATCH) {
-      int lo = 0, hi = a.njobs - 1;  // last job whose first chunk id is <= t (empty jobs are skipped)
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (cb[mid] <= t) lo = mid;
-        else hi = mid - 1;
-      }
+      const int lo = job_of(t);
       const BatchJob& j = a.jobs[lo];
       seg = cb[lo];
       job = lo;
@@ -626,15 +650,16 @@ __global__ void __launch_bounds__((NW + 1) * 32, MINB)
       fence_proxy_async_smem();
       __syncwarp();
     }
-    if constexpr (!BATCH) {
-      // The chunk about a full round of tickets ahead goes to L2, so that its warp's
-      // load takes one L2 round trip, not a queue at HBM that all later chunks' places
-      // would wait for.  After the pack, not before: at a kernel's start the first
-      // loads of all warps are still under way (302 MB f64 lossless: 108 us against 116
-      // with the prefetch right after the load and 110 without one).
-      const long long ahead = t + static_cast<long long>(gridDim.x) * NW;
-      if (lane == 0 && (ahead + 1) * CS <= a.insize && (reinterpret_cast<uintptr_t>(a.in) & 15u) == 0u)
-        prefetch_l2(a.in + ahead * CS, CS);
+    // The chunk about a full round of tickets ahead goes to L2, so that its warp's load
+    // takes one L2 round trip, not a queue at HBM that all later chunks' places would
+    // wait for.  After the pack, not before: at a kernel's start the first loads of all
+    // warps are still under way (302 MB f64 lossless: 108 us against 116 with the
+    // prefetch right after the load and 110 without one; batch of 60 arrays: 65.3
+    // against 67.5 without one).
+    const long long ahead = t + static_cast<long long>(gridDim.x) * NW;
+    if (ahead < total) {
+      const uint8_t* in = whole_chunk(ahead);
+      if (lane == 0 && in != nullptr) prefetch_l2(in, CS);
     }
     long long excl = scan.prefix(k.g, BATCH && k.c > 0 ? seg : 0, hdr);
     if constexpr (BATCH) {
