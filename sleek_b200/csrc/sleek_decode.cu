@@ -571,9 +571,10 @@ __global__ void __launch_bounds__(DB_NT, 1) k_decode_batch(const BatchDecArgs a)
   }
   grid_wait();
   for (int i = tid; i <= a.njobs; i += DB_NT) cb[i] = a.chunk_base[i];
-  __syncthreads();
+  // the prepass found an error (one thread looks: another CTA may report one meanwhile,
+  // and a team's warps have to agree)
+  const bool failed_before = __syncthreads_or(tid == 0 && ld_relaxed_u64(&ws[WS_STATUS]) != 0ull) != 0;
   const long long total = cb[a.njobs];
-  const bool failed_before = ld_relaxed_u64(&ws[WS_STATUS]) != 0ull;  // the prepass found an error
   uint8_t* const stg = smem + team * DEC_STAGE;
   uint64_t* const bar = &bars[team];
   uint32_t par = 0;
