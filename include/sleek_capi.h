@@ -5,7 +5,7 @@
  * include/sleek_lossy_gpu.h of SLEEK).  Plain pointers and sizes only; every entry
  * point is asynchronous on the given CUDA stream (NULL = legacy default stream) and
  * returns a status code for everything it can check on the host.  Errors found on
- * the device (malformed stream, a look-back wait that exceeded its time limit)
+ * the device (malformed stream, a wait that exceeded its time limit)
  * never trap: the kernel writes -status into the size output (*d_encsize or
  * *d_decsize), and the status is also readable with sleek_workspace_status().
  *
@@ -15,7 +15,7 @@
  *
  * Pointers: device inputs/outputs must be aligned to their element size (4 for
  * float, 8 for double); the stream buffer must be 8-byte aligned.  16-byte
- * aligned inputs take the TMA path; others are loaded with ordinary loads.
+ * aligned inputs take the TMA path; others are copied 4 bytes at a time.
  *
  * Workspace: pass NULL to use a workspace the library owns (one per device and
  * stream, grown on demand -- growth calls cudaMalloc, so size it up front with a
@@ -150,8 +150,10 @@ int sleek_compress_f32_static(const float* d_input, long long num_elements, unsi
 int sleek_set_ctas_per_sm(int decompress, int elem_bytes, int lossy, int ctas_per_sm);
 
 /* Tuning: launch shapes.  The single-buffer kernels are built in a few shapes (threads per
- * CTA, compute warps, shared-memory chunk stages, and the CTAs per SM their registers are
- * budgeted for); shape 0 is the default, and every shape writes the same bytes.
+ * CTA, warps that work on chunks, shared-memory chunk stages, and the CTAs per SM their
+ * registers are budgeted for); shape 0 is the default -- with as many CTAs as fit it also
+ * stands for the kernels' small-input forms, by the number of chunks -- and every shape
+ * writes the same bytes.
  * sleek_launch_shape_info describes shape `shape` of the compress (decompress = 0) or
  * decompress kernels (any output pointer may be NULL) and returns SLEEK_ERR_INVALID_ARG
  * past the last one.  sleek_set_launch_shape selects the shape and the CTAs per SM (0 = as
@@ -332,9 +334,9 @@ const char* sleek_stream_reason_string(int reason);
 
 /* Self-test of the device-side time limits (no counterpart in the reference, whose
  * waits are unbounded): a one-warp kernel waits on an mbarrier that nothing arrives
- * on and looks back over a predecessor flag that nothing publishes, each limited to
+ * on and for the size of a preceding chunk that nothing publishes, each limited to
  * limit_ns (0 < limit_ns <= 10 s), with the same wait helpers as the codec kernels.
- * h_result[0] = 1 if the barrier wait gave up, h_result[1] = the look-back's result
+ * h_result[0] = 1 if the barrier wait gave up, h_result[1] = the second wait's result
  * (-1 when it gave up), h_result[2] = nanoseconds both waits took.  Synchronous on
  * the legacy default stream; the device stays usable. */
 int sleek_selftest_bounded_waits(long long limit_ns, long long* h_result);

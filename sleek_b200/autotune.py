@@ -6,8 +6,8 @@ laid on the GPU, where the reference uses fixed constants (``SLEEK_TPB`` = 512
 threads and a grid from ``sleek_thread_blocks``, include/sleek_common_gpu.h:54-56,
 108-119):
 
-- single-buffer calls: the kernel shape -- threads per CTA, compute warps (and so
-  subchunks per warp) and shared-memory chunk stages, from the shapes the library
+- single-buffer calls: the kernel shape -- warps that work on chunks, and
+  shared-memory chunk stages, from the shapes the library
   is built with (``sleek_launch_shape_info``) -- and the CTAs per SM, per kind
   (element size, lossless / lossy, compress / decompress) and per input-size
   bucket (base-2 logarithm of the bytes), applied with ``sleek_set_launch_shape``;

@@ -3,7 +3,7 @@ float64 and mixed error bounds in one persistent launch (per group of up to 1024
 arrays), optionally captured in a CUDA graph.
 
 Each array's stream is bit-identical to what ``sleek_compress_gpu`` produces for
-it alone; the batched look-back is segmented per array.
+it alone; a chunk's place is relative to its array's first chunk.
 
     plan = BatchPlan.compress(arrays, error_bounds)    # validates, uploads tables
     plan.run()                                          # or plan.graph().replay()

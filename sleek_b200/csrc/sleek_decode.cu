@@ -8,10 +8,10 @@
 // stores.  No CTA waits for another, and there is no CTA barrier per chunk.  Malformed
 // streams set an error status instead of trapping; every wait is bounded.
 //
-// What bounds it: HBM on large fields (302 MB f64 at eb 1e-4: 73.4 -> 65.5 us, 0.93 of
-// the measured copy rate without the launch), else the waits at the start (header and
-// table, the first chunks' copies) and the ALU pipe (26 MB f32 at eb 1e-3: 18.2 ->
-// 14.3 us; 67 MB f32 lossless: 30.1 -> 28.7 us; batch of 60 arrays: 60.0 -> 55.5 us).
+// What bounds it: HBM on large fields (302 MB f64 at eb 1e-4: 73.0 -> 63.6 us, 0.91 of
+// the measured copy rate), else the waits at the start (header and table, the first
+// chunks' copies) and the ALU pipe (26 MB f32 at eb 1e-3: 18.2 -> 11.5 us; 67 MB f32
+// lossless: 29.7 -> 26.5 us; batch of 60 arrays: 60.7 -> 50.4 us).
 // A chunk costs 1,300 warp instructions (f64, eb 1e-4), 2,720 when eight warps shared
 // it and each lane took every 32nd value.
 #include <type_traits>

@@ -17,8 +17,8 @@
 // bytes to their place), and its stage is taken for 8-10 us.  Every wait between the
 // published size and the store counts against the stages, so the pack comes before
 // the wait for the place, at the alignment the place is expected to have.
-// (302 MB f64 field: lossless 144 -> 114 us, eb 1e-4 129 -> 90 us; 26 MB f32 field,
-// eb 1e-3: 24.1 -> 16.7 us; 67 MB f32 signal, lossless: 44.6 -> 34.8 us.)
+// (302 MB f64 field: lossless 144 -> 111 us, eb 1e-4 130 -> 89 us; 26 MB f32 field,
+// eb 1e-3: 24.1 -> 12.9 us; 67 MB f32 signal, lossless: 44.6 -> 31.8 us.)
 #include <type_traits>
 
 #include "sleek_device.cuh"
