@@ -182,11 +182,16 @@ __device__ __forceinline__ bool decode_chunk(const uint8_t* stg, int sft, int cs
         for (int u = 0; u < DEC_G; ++u) e[u] = codes_narrow<B>(w, b[u], l[u], lane);
 #pragma unroll
         for (int u = 0; u < DEC_G; ++u) put(i0 + u, decode_codes<T, LOSSY, true>(e[u], q));
-      } else if (wm == ALL && (B == 8 || !LOSSY || pm == ALL)) {
+      } else if (wm == ALL) {
 #pragma unroll
         for (int u = 0; u < DEC_G; ++u) e[u] = codes_wide<B>(w, b[u], l[u], lane);
+        if (B == 4 && LOSSY && pm == ALL) {
 #pragma unroll
-        for (int u = 0; u < DEC_G; ++u) put(i0 + u, decode_codes<T, LOSSY, B == 4>(e[u], q));
+          for (int u = 0; u < DEC_G; ++u) put(i0 + u, decode_codes<T, LOSSY, true>(e[u], q));
+        } else {
+#pragma unroll
+          for (int u = 0; u < DEC_G; ++u) put(i0 + u, decode_codes<T, LOSSY, false>(e[u], q));
+        }
       } else {
 #pragma unroll
         for (int u = 0; u < DEC_G; ++u) {
