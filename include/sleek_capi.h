@@ -341,6 +341,19 @@ const char* sleek_stream_reason_string(int reason);
  * the legacy default stream; the device stays usable. */
 int sleek_selftest_bounded_waits(long long limit_ns, long long* h_result);
 
+/* Self-test of the encoder's placing of chunks (no counterpart in the reference).
+ * sleek_selftest_chunk_scan publishes `chunks` compressed sizes (1 .. 16384 each) on the
+ * device, lets a scanner walk over them, and asks for the places of the `n` chunks
+ * h_index: h_prefix[i] receives the sum of the sizes before chunk h_index[i] (-1 if the
+ * wait for it gave up), whether or not the scanner's ring still holds its group.
+ * *h_uneven receives how many lanes got another alignment hint than their warp's first
+ * lane when they asked one after the other while the ring moved (0).  Synchronous on the
+ * legacy default stream.  sleek_selftest_ring_holds (host only) is 1 if the ring's entry
+ * of `group`, read before the scanner had `known` groups, cannot have been overwritten. */
+int sleek_selftest_chunk_scan(const unsigned* h_sizes, long long chunks, const long long* h_index, int n,
+                              long long* h_prefix, unsigned* h_uneven);
+int sleek_selftest_ring_holds(long long known, long long group);
+
 /* Self-test of the device value maps (no counterpart in the reference): on the current
  * device, compares what the codec kernels compute -- the lossless transform and its
  * inverse, quantize and dequantize (whose rounding division runs in floating point) --

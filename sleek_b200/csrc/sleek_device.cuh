@@ -631,6 +631,14 @@ struct ScanRing {
   int gone;             // warps that have left their chunk loop
 };
 
+// Whether the entry of group `own`, read before `known`, was still its own: with
+// `known` groups known the scanner is at most writing the 32 after them.
+__host__ __device__ constexpr bool ring_holds(long long known, long long own) { return known + 32 < own + RING; }
+
+// The ring and the count of warps that have left change while they are read, and the
+// lanes of a warp need not read them at the same time.  So the warp goes on with what
+// lane 0 saw: the alignment a chunk is packed at and the branches around warp-wide
+// exchanges have to be the same in all lanes.
 struct ChunkScan {
   uint32_t* flags;  // per chunk
   uint64_t* sums;   // per group: sum of sizes | count << 32
@@ -672,7 +680,7 @@ struct ChunkScan {
     const long long last = (chunks + GROUP - 1) / GROUP - 1;
     long long f = 0;
     uint64_t before = 0;
-    while (f < last && ring->gone < warps) {
+    while (f < last && __any_sync(0xffffffffu, lane == 0 && ring->gone < warps)) {
       const long long h = f + lane;
       const uint64_t v = h < last ? ld_relaxed_u64(sums + h) : 0ull;
       const unsigned no = __ballot_sync(0xffffffffu, (v >> 32) != GROUP);
@@ -693,14 +701,16 @@ struct ChunkScan {
     }
   }
 
-  // The prefix before chunk `idx`, modulo 8 or 16, if every chunk after the last
-  // group known so far is compressed (size 2 modulo that); a hint only.
-  __device__ long long guess(long long idx) const
+  // One warp: the prefix before chunk `idx`, modulo 8 or 16, if every chunk after the
+  // last group known so far is compressed (size 2 modulo that); a hint only, but the
+  // same in every lane.
+  __device__ int guess(long long idx) const
   {
     const long long own = idx / GROUP;
     long long g = ring->known;
     g = g < own ? g : own;
-    return (g > 0 ? static_cast<long long>(ring->base[g % RING]) : 0ll) + 2 * (idx - g * GROUP);
+    const long long v = (g > 0 ? static_cast<long long>(ring->base[g % RING]) : 0ll) + 2 * (idx - g * GROUP);
+    return __shfl_sync(0xffffffffu, static_cast<int>(v), 0);
   }
 
   // One warp: the sum of the sizes of all chunks before `idx`, or -1 when a wait
@@ -730,11 +740,13 @@ struct ChunkScan {
           need_own = false;
         }
       }
-      if (need_base && ring->known >= own) {
+      if (need_base && __any_sync(0xffffffffu, lane == 0 && ring->known >= own)) {
         __threadfence_block();
         uint64_t v = ring->base[own % RING];
         __threadfence_block();
-        if (ring->known + 32 >= own + RING) {  // the entry may be gone: add up the groups
+        if (__any_sync(0xffffffffu, lane == 0 && ring_holds(ring->known, own))) {
+          v = __shfl_sync(0xffffffffu, v, 0);
+        } else {  // the entry may be gone: add up the groups
           uint64_t s = 0;
           for (long long h = lane; h < own; h += 32) s += ld_relaxed_u64(sums + h) & 0xffffffffull;
           v = static_cast<uint64_t>(warp_sum(static_cast<long long>(s)));

@@ -6,6 +6,10 @@
 // wait helpers as the encode and decode kernels (sleek_device.cuh).  Both must
 // give up, report it, and return; the context stays usable.
 //
+// Chunk scan: the encoder's placing of chunks (ChunkScan) on given sizes, for chunks whose
+// group is in the scanner's ring and for those whose entry the ring has lost, and its
+// alignment hint read by lanes that arrive one after the other while the ring moves.
+//
 // Value maps: the transforms, quantizers and dequantizers the kernels compute
 // (sleek_device.cuh, rewritten forms) against a literal restatement of the
 // reference's integer steps, over every 32-bit word and over every 64-bit
@@ -43,6 +47,72 @@ __global__ void __launch_bounds__(32) k_selftest_waits(unsigned long long limit_
     result[0] = got ? 0 : 1;
     result[1] = lb;
     result[2] = static_cast<long long>(t1 - t0);
+  }
+}
+
+__global__ void __launch_bounds__(256) k_selftest_publish(uint64_t* region, long long chunks, const uint32_t* sizes)
+{
+  const ChunkScan scan(region, chunks, nullptr);
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < chunks; i += gridDim.x * 256ll) scan.publish(i, sizes[i]);
+}
+
+// One warp: the scanner's walk over all groups, then the places of chunks `index`.
+__global__ void __launch_bounds__(32) k_selftest_places(uint64_t* region, long long chunks, const uint64_t* hdr,
+                                                        const long long* index, int n, long long* prefix)
+{
+  __shared__ ScanRing ring;
+  if (threadIdx.x == 0) {
+    ring.known = 0;
+    ring.gone = 0;
+  }
+  __syncwarp();
+  const ChunkScan scan(region, chunks, &ring);
+  scan.follow(1);
+  __syncwarp();
+  for (int i = 0; i < n; ++i) {
+    const long long p = scan.prefix(index[i], 0, hdr);
+    if (threadIdx.x == 0) prefix[i] = p;
+  }
+}
+
+// Warp 1 moves the ring on while the lanes of warp 0, each some 1,000 clocks after the
+// one before it, ask for the same chunk's hint: `uneven` counts the answers that are not
+// lane 0's.
+__global__ void __launch_bounds__(64) k_selftest_hint(int rounds, unsigned* uneven)
+{
+  __shared__ ScanRing ring;
+  __shared__ volatile int done;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    ring.known = 0;
+    ring.gone = 0;
+    done = 0;
+  }
+  __syncthreads();
+  const long long chunks = 1ll << 40;  // (only the ring is used)
+  const ChunkScan scan(nullptr, chunks, &ring);
+  if (threadIdx.x >= 32) {
+    if (lane == 0) {
+      volatile ScanRing* const r = &ring;
+      for (long long g = 1; g < 100000 && !done; ++g) {
+        r->base[g % RING] = static_cast<uint64_t>(3 * g);
+        __threadfence_block();
+        r->known = g;
+        __nanosleep(100);
+      }
+    }
+  } else {
+    unsigned bad = 0;
+    for (int i = 0; i < rounds; ++i) {
+      const long long t0 = clock64();
+      while (clock64() - t0 < 1000ll * lane) {
+      }
+      const int v = scan.guess(chunks - 1);
+      bad += v != __shfl_sync(0xffffffffu, v, 0);
+    }
+    atomicAdd(uneven, bad);
+    __syncwarp();
+    if (lane == 0) done = 1;
   }
 }
 
@@ -288,6 +358,56 @@ extern "C" int sleek_selftest_bounded_waits(long long limit_ns, long long* h_res
   }
   cudaFree(d);
   cudaFree(d_res);
+  if (rc) cudaGetLastError();
+  return rc;
+}
+
+extern "C" int sleek_selftest_ring_holds(long long known, long long group) { return sleek::ring_holds(known, group); }
+
+extern "C" int sleek_selftest_chunk_scan(const unsigned* h_sizes, long long chunks, const long long* h_index, int n,
+                                         long long* h_prefix, unsigned* h_uneven)
+{
+  if (!h_sizes || !h_index || !h_prefix || !h_uneven || chunks < 1 || chunks > (1ll << 24) || n < 1 || n > 65536)
+    return SLEEK_ERR_INVALID_ARG;
+  for (long long i = 0; i < chunks; ++i)
+    if (h_sizes[i] < 1 || h_sizes[i] > sleek::CS) return SLEEK_ERR_INVALID_ARG;
+  for (int i = 0; i < n; ++i)
+    if (h_index[i] < 0 || h_index[i] >= chunks) return SLEEK_ERR_INVALID_ARG;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return SLEEK_ERR_NO_DEVICE;
+  }
+  const size_t region = 8 * static_cast<size_t>(sleek::WS_HDR_WORDS + sleek::scan_words(chunks));
+  uint64_t* d = nullptr;  // header, then flags and sums
+  uint32_t* d_sizes = nullptr;
+  long long* d_index = nullptr;  // the indexes, then the places
+  unsigned* d_uneven = nullptr;
+  int rc = SLEEK_OK;
+  if (cudaMalloc(&d, region) != cudaSuccess || cudaMalloc(&d_sizes, 4 * static_cast<size_t>(chunks)) != cudaSuccess ||
+      cudaMalloc(&d_index, 16 * static_cast<size_t>(n)) != cudaSuccess || cudaMalloc(&d_uneven, 4) != cudaSuccess ||
+      cudaMemset(d, 0, region) != cudaSuccess || cudaMemset(d_uneven, 0, 4) != cudaSuccess ||
+      cudaMemcpy(d_sizes, h_sizes, 4 * static_cast<size_t>(chunks), cudaMemcpyHostToDevice) != cudaSuccess ||
+      cudaMemcpy(d_index, h_index, 8 * static_cast<size_t>(n), cudaMemcpyHostToDevice) != cudaSuccess) {
+    rc = SLEEK_ERR_CUDA;
+  } else {
+    uint64_t* const flags = d + sleek::WS_HDR_WORDS;
+    sleek::k_selftest_publish<<<64, 256>>>(flags, chunks, d_sizes);
+    bool ok = cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
+    if (ok) {  // every size is published: the scanner's walk ends
+      sleek::k_selftest_places<<<1, 32>>>(flags, chunks, d, d_index, n, d_index + n);
+      sleek::k_selftest_hint<<<1, 64>>>(32, d_uneven);
+      ok = cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
+    }
+    if (!ok ||
+        cudaMemcpy(h_prefix, d_index + n, 8 * static_cast<size_t>(n), cudaMemcpyDeviceToHost) != cudaSuccess ||
+        cudaMemcpy(h_uneven, d_uneven, 4, cudaMemcpyDeviceToHost) != cudaSuccess)
+      rc = SLEEK_ERR_CUDA;
+  }
+  cudaFree(d);
+  cudaFree(d_sizes);
+  cudaFree(d_index);
+  cudaFree(d_uneven);
   if (rc) cudaGetLastError();
   return rc;
 }
