@@ -341,6 +341,14 @@ const char* sleek_stream_reason_string(int reason);
  * the legacy default stream; the device stays usable. */
 int sleek_selftest_bounded_waits(long long limit_ns, long long* h_result);
 
+/* Self-test of single device waits, each limited to limit_ns (0 < limit_ns <= 1 s), run
+ * out or not as `what` says; h_result[0] is what the wait led to, h_result[2] the
+ * nanoseconds it took.
+ *   0, 1  a decode team of two warps of which warp 0 or 1 gives up and the other does not:
+ *         the status they report (SLEEK_ERR_TIMEOUT), at position h_result[1] (7)
+ * Synchronous on the legacy default stream; the device stays usable. */
+int sleek_selftest_wait(int what, long long limit_ns, long long* h_result);
+
 /* Self-test of the encoder's placing of chunks (no counterpart in the reference).
  * sleek_selftest_chunk_scan publishes `chunks` compressed sizes (1 .. 16384 each) on the
  * device, lets a scanner walk over them, and asks for the places of the `n` chunks

@@ -92,6 +92,7 @@ SIGNATURES = {
     "sleek_validate_stream": (C.c_int, [_vp, C.c_longlong, C.c_int, _vp]),
     "sleek_stream_reason_string": (C.c_char_p, [C.c_int]),
     "sleek_selftest_bounded_waits": (C.c_int, [C.c_longlong, C.POINTER(C.c_longlong)]),
+    "sleek_selftest_wait": (C.c_int, [C.c_int, C.c_longlong, C.POINTER(C.c_longlong)]),
     "sleek_selftest_chunk_scan": (C.c_int, [_vp, _i64, _vp, C.c_int, _vp, C.POINTER(C.c_uint)]),
     "sleek_selftest_ring_holds": (C.c_int, [_i64, _i64]),
     "sleek_selftest_value_maps": (C.c_int, [C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)]),

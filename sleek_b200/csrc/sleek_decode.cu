@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(NTEAM * TW * 32, MINB) k_decode(const DecArgs 
         uint8_t* const dst = a.out + c * CS;
         if (!late) ok = decode_chunk<T, LOSSY, TW>(stg + cur.pos, cur.sft, cur.cs, osize, dst, a.q, cw, lane);
       }
-      if (lane == 0 && cw == 0 && (late || !ok)) set_status(hdr, late ? ST_TIMEOUT : ST_CORRUPT, c);
+      report_chunk(hdr, late, ok, cw, lane, c);
       // the stage is read before it is refilled (generic accesses ordered before the TMA write)
       fence_proxy_async_smem();
       left = team_failed<TW>(team, late);
@@ -650,15 +650,13 @@ __global__ void __launch_bounds__(DB_NT, 1) k_decode_batch(const BatchDecArgs a)
       uint8_t* const out = cur.out + cur.c * CS;
       const int osize = static_cast<int>(min(static_cast<long long>(CS), cur.insize - cur.c * CS));
       bool ok = true;
-      if (late) {
-        if (lane == 0) set_status(ws, ST_TIMEOUT, ct);
-      } else switch (cur.kind) {
+      if (!late) switch (cur.kind) {
         case 0: ok = decode_chunk<uint32_t, false, DB_TW>(stg, sft, cs, osize, out, cur.q, cw, lane); break;
         case 1: ok = decode_chunk<uint64_t, false, DB_TW>(stg, sft, cs, osize, out, cur.q, cw, lane); break;
         case 2: ok = decode_chunk<uint32_t, true, DB_TW>(stg, sft, cs, osize, out, cur.q, cw, lane); break;
         default: ok = decode_chunk<uint64_t, true, DB_TW>(stg, sft, cs, osize, out, cur.q, cw, lane); break;
       }
-      if (!ok && leads) set_status(ws, ST_CORRUPT, ct);
+      report_chunk(ws, late, ok, cw, lane, ct);
       // the stage is read before it is refilled (generic accesses ordered before the TMA write)
       fence_proxy_async_smem();
       if (team_failed<DB_TW>(team, late)) break;

@@ -204,6 +204,14 @@ __device__ __forceinline__ void set_status(uint64_t* hdr, unsigned code, long lo
   }
 }
 
+// What became of a chunk that a team of warps decoded: each warp (`cw` of its team)
+// reports its own wait that gave up, since the others' may have ended well; what is
+// wrong with the chunk itself they all see, so the first reports it.
+__device__ __forceinline__ void report_chunk(uint64_t* hdr, bool late, bool ok, int cw, int lane, long long pos)
+{
+  if (lane == 0 && (late || (!ok && cw == 0))) set_status(hdr, late ? ST_TIMEOUT : ST_CORRUPT, pos);
+}
+
 // ----------------------------------------------------------------------------
 // Self-resetting workspace of the single-buffer kernels.  A launch works in
 // result block and flag region p = epoch & 1 (both clean when it starts), and

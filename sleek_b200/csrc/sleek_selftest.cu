@@ -50,6 +50,32 @@ __global__ void __launch_bounds__(32) k_selftest_waits(unsigned long long limit_
   }
 }
 
+// Two warps as a decode team: the wait of warp `what` (0 or 1) gives up, the other's
+// ends well.  result[0]: the status that the team leaves in `hdr`; result[1]: the
+// position; result[2]: nanoseconds
+__global__ void __launch_bounds__(64) k_selftest_team(int what, unsigned long long limit_ns, uint64_t* hdr,
+                                                      long long* result)
+{
+  __shared__ __align__(8) uint64_t bars[2];
+  const int lane = threadIdx.x & 31, cw = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    mbar_fence_init();
+    mbar_arrive(&bars[1 - what]);
+  }
+  __syncthreads();
+  const unsigned long long t0 = globaltimer_ns();
+  const bool late = __any_sync(0xffffffffu, !mbar_wait_bounded(&bars[cw], 0, limit_ns));
+  report_chunk(hdr, late, true, cw, lane, 7);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    result[0] = static_cast<long long>(ld_relaxed_u64(&hdr[WS_STATUS]));
+    result[1] = static_cast<long long>(ld_relaxed_u64(&hdr[WS_ERRPOS]));
+    result[2] = static_cast<long long>(globaltimer_ns() - t0);
+  }
+}
+
 __global__ void __launch_bounds__(256) k_selftest_publish(uint64_t* region, long long chunks, const uint32_t* sizes)
 {
   const ChunkScan scan(region, chunks, nullptr);
@@ -352,6 +378,33 @@ extern "C" int sleek_selftest_bounded_waits(long long limit_ns, long long* h_res
     rc = SLEEK_ERR_CUDA;
   } else {
     sleek::k_selftest_waits<<<1, 32>>>(static_cast<unsigned long long>(limit_ns), d, d_res);
+    if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
+        cudaMemcpy(h_result, d_res, 3 * sizeof(long long), cudaMemcpyDeviceToHost) != cudaSuccess)
+      rc = SLEEK_ERR_CUDA;
+  }
+  cudaFree(d);
+  cudaFree(d_res);
+  if (rc) cudaGetLastError();
+  return rc;
+}
+
+extern "C" int sleek_selftest_wait(int what, long long limit_ns, long long* h_result)
+{
+  if (!h_result || what < 0 || what > 1 || limit_ns <= 0 || limit_ns > 1000000000ll) return SLEEK_ERR_INVALID_ARG;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return SLEEK_ERR_NO_DEVICE;
+  }
+  uint64_t* d = nullptr;  // a zeroed workspace header
+  long long* d_res = nullptr;
+  int rc = SLEEK_OK;
+  if (cudaMalloc(&d, sleek::WS_HDR_WORDS * sizeof(uint64_t)) != cudaSuccess ||
+      cudaMalloc(&d_res, 3 * sizeof(long long)) != cudaSuccess ||
+      cudaMemset(d, 0, sleek::WS_HDR_WORDS * sizeof(uint64_t)) != cudaSuccess) {
+    rc = SLEEK_ERR_CUDA;
+  } else {
+    sleek::k_selftest_team<<<1, 64>>>(what, static_cast<unsigned long long>(limit_ns), d, d_res);
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
         cudaMemcpy(h_result, d_res, 3 * sizeof(long long), cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = SLEEK_ERR_CUDA;
