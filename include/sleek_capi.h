@@ -346,6 +346,8 @@ int sleek_selftest_bounded_waits(long long limit_ns, long long* h_result);
  * nanoseconds it took.
  *   0, 1  a decode team of two warps of which warp 0 or 1 gives up and the other does not:
  *         the status they report (SLEEK_ERR_TIMEOUT), at position h_result[1] (7)
+ *   2     a bulk copy that does not land: 0 (not landed), after the limit and, because the
+ *         warp would leave, a second wait as long
  * Synchronous on the legacy default stream; the device stays usable. */
 int sleek_selftest_wait(int what, long long limit_ns, long long* h_result);
 

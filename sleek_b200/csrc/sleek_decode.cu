@@ -443,9 +443,8 @@ __global__ void __launch_bounds__(NTEAM * TW * 32, MINB) k_decode(const DecArgs 
       bool late = false;
       bool ok = cur.cs > 0;
       if (ok) {
-        const bool got = mbar_wait_bounded(&bar[slot], (par >> slot) & 1u);
+        late = !copy_landed(&bar[slot], (par >> slot) & 1u);
         par ^= 1u << slot;
-        late = __any_sync(0xffffffffu, !got);
         const int osize = static_cast<int>(min(static_cast<long long>(CS), insize - c * CS));
         uint8_t* const dst = a.out + c * CS;
         if (!late) ok = decode_chunk<T, LOSSY, TW>(stg + cur.pos, cur.sft, cur.cs, osize, dst, a.q, cw, lane);
@@ -644,9 +643,8 @@ __global__ void __launch_bounds__(DB_NT, 1) k_decode_batch(const BatchDecArgs a)
     t = drawn();
     if (t < total) it = look_up(t);
     if (cs > 0) {
-      const bool got = mbar_wait_bounded(bar, par);
+      const bool late = !copy_landed(bar, par);
       par ^= 1u;
-      const bool late = __any_sync(0xffffffffu, !got);
       uint8_t* const out = cur.out + cur.c * CS;
       const int osize = static_cast<int>(min(static_cast<long long>(CS), cur.insize - cur.c * CS));
       bool ok = true;

@@ -122,6 +122,18 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return true;
 }
 
+// One warp: the bulk copy counted on `bar` has landed.  False if it has not within
+// `limit_ns`; then the warp, which is about to leave, has waited for it once more, so
+// that it does not land in shared memory that belongs to another CTA by then.
+__device__ __forceinline__ bool copy_landed(uint64_t* bar, uint32_t parity,
+                                            unsigned long long limit_ns = SPIN_TIMEOUT_NS)
+{
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k)
+    if (__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, limit_ns))) return k == 0;
+  return false;
+}
+
 // 1-D bulk copy global -> shared (no multicast); completion counted on `bar`.
 __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar)
 {

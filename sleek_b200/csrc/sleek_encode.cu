@@ -472,9 +472,9 @@ __device__ __forceinline__ bool load_chunk(uint8_t* dst, const uint8_t* in, int 
       mbar_arrive_expect_tx(bar, CS);
       tma_load_1d(dst, in, CS, bar);
     }
-    const bool ok = mbar_wait_bounded(bar, par);
+    const bool ok = copy_landed(bar, par);
     par ^= 1u;
-    return !__any_sync(0xffffffffu, !ok);
+    return ok;
   }
   auto copy = [&](auto width) {
     constexpr int N = decltype(width)::value;
@@ -785,13 +785,13 @@ __global__ void __launch_bounds__(ENC_TEAM * 32, ENC_TEAM_CTAS) k_encode_team(co
     const uint8_t* const in = a.in + c * CS;
     const int osize = static_cast<int>(min(static_cast<long long>(CS), a.insize - c * CS));
     const unsigned mis = static_cast<unsigned>(reinterpret_cast<uintptr_t>(in)) & 15u;
-    bool late = false;
+    bool wlate = false;
     if (mis == 0u && osize == CS) {
       if (tid == 0) {
         mbar_arrive_expect_tx(&bar, CS);
         tma_load_1d(stg, in, CS, &bar);
       }
-      late = !mbar_wait_bounded(&bar, 0);
+      wlate = !copy_landed(&bar, 0);
     } else {  // a warp's own subchunks, zero-padded
       for (int k = 0; k < EW_G * 4; ++k) {
         const int o = (warp * EW_G * 4 + k) * 128 + lane * 4;
@@ -801,7 +801,6 @@ __global__ void __launch_bounds__(ENC_TEAM * 32, ENC_TEAM_CTAS) k_encode_team(co
       cp_async_wait_all();
       __syncwarp();
     }
-    const bool wlate = __any_sync(0xffffffffu, late);
     uint4 w[EW_G];
     int width = 0;
     if (!wlate) width = encode_group<KIND, false, false>(stg, w, warp * EW_G, a.q, lane);

@@ -50,6 +50,26 @@ __global__ void __launch_bounds__(32) k_selftest_waits(unsigned long long limit_
   }
 }
 
+// One warp waits for a copy that never lands.  result[0]: 1 if it is told that it has;
+// result[2]: nanoseconds
+__global__ void __launch_bounds__(32) k_selftest_copy(unsigned long long limit_ns, long long* result)
+{
+  __shared__ __align__(8) uint64_t bar;
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 1);
+    mbar_fence_init();
+  }
+  __syncwarp();
+  const unsigned long long t0 = globaltimer_ns();
+  const bool landed = copy_landed(&bar, 0, limit_ns);
+  const unsigned long long t1 = globaltimer_ns();
+  if (threadIdx.x == 0) {
+    result[0] = landed;
+    result[1] = 0;
+    result[2] = static_cast<long long>(t1 - t0);
+  }
+}
+
 // Two warps as a decode team: the wait of warp `what` (0 or 1) gives up, the other's
 // ends well.  result[0]: the status that the team leaves in `hdr`; result[1]: the
 // position; result[2]: nanoseconds
@@ -390,7 +410,7 @@ extern "C" int sleek_selftest_bounded_waits(long long limit_ns, long long* h_res
 
 extern "C" int sleek_selftest_wait(int what, long long limit_ns, long long* h_result)
 {
-  if (!h_result || what < 0 || what > 1 || limit_ns <= 0 || limit_ns > 1000000000ll) return SLEEK_ERR_INVALID_ARG;
+  if (!h_result || what < 0 || what > 2 || limit_ns <= 0 || limit_ns > 1000000000ll) return SLEEK_ERR_INVALID_ARG;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
     cudaGetLastError();
@@ -404,7 +424,9 @@ extern "C" int sleek_selftest_wait(int what, long long limit_ns, long long* h_re
       cudaMemset(d, 0, sleek::WS_HDR_WORDS * sizeof(uint64_t)) != cudaSuccess) {
     rc = SLEEK_ERR_CUDA;
   } else {
-    sleek::k_selftest_team<<<1, 64>>>(what, static_cast<unsigned long long>(limit_ns), d, d_res);
+    const unsigned long long limit = static_cast<unsigned long long>(limit_ns);
+    if (what < 2) sleek::k_selftest_team<<<1, 64>>>(what, limit, d, d_res);
+    else sleek::k_selftest_copy<<<1, 32>>>(limit, d_res);
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
         cudaMemcpy(h_result, d_res, 3 * sizeof(long long), cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = SLEEK_ERR_CUDA;

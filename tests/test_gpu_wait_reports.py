@@ -22,3 +22,9 @@ def test_every_warp_of_a_team_reports_its_own_timeout(cuda, warp):
     status, pos, ns = run(warp)
     assert (status, pos) == (_capi.SLEEK_ERR_TIMEOUT, 7)
     assert ns >= LIMIT
+
+
+def test_a_warp_waits_once_more_for_its_copy_before_it_leaves(cuda):
+    landed, _, ns = run(2)
+    assert landed == 0
+    assert ns >= 2 * LIMIT
