@@ -348,6 +348,9 @@ int sleek_selftest_bounded_waits(long long limit_ns, long long* h_result);
  *         the status they report (SLEEK_ERR_TIMEOUT), at position h_result[1] (7)
  *   2     a bulk copy that does not land: 0 (not landed), after the limit and, because the
  *         warp would leave, a second wait as long
+ *   3     a chunk whose group the encoder's scanner never reaches: -1
+ *   4     a preceding chunk of a small input that is never sized: -1
+ *   5     a batched buffer whose start is never told: 0
  * Synchronous on the legacy default stream; the device stays usable. */
 int sleek_selftest_wait(int what, long long limit_ns, long long* h_result);
 

@@ -788,7 +788,8 @@ struct ChunkScan {
   }
 
   // One warp: the same from the flags alone, for a few groups, with no scanner.
-  __device__ long long prefix_flags(long long idx, const uint64_t* hdr) const
+  __device__ long long prefix_flags(long long idx, const uint64_t* hdr,
+                                    unsigned long long limit_ns = SPIN_TIMEOUT_NS) const
   {
     const int lane = threadIdx.x & 31;
     long long excl = 0;
@@ -805,7 +806,7 @@ struct ChunkScan {
         if (++polls == 256) {
           t0 = globaltimer_ns();
         } else if (polls > 256 && (polls & 255) == 0) {
-          const bool late = globaltimer_ns() - t0 > SPIN_TIMEOUT_NS;
+          const bool late = globaltimer_ns() - t0 > limit_ns;
           const bool failed = ld_relaxed_u64(&hdr[WS_STATUS]) != 0ull;
           if (__any_sync(0xffffffffu, late || failed)) return -1;
         }
@@ -816,7 +817,7 @@ struct ChunkScan {
   }
 
   // One warp: the value another warp puts at `p` (never 0), or 0 when the wait gave up.
-  __device__ static uint64_t await(const uint64_t* p, const uint64_t* hdr)
+  __device__ static uint64_t await(const uint64_t* p, const uint64_t* hdr, unsigned long long limit_ns = SPIN_TIMEOUT_NS)
   {
     unsigned long long t0 = 0;
     for (int polls = 0;; ++polls) {
@@ -825,7 +826,7 @@ struct ChunkScan {
       if (polls == 256) {
         t0 = globaltimer_ns();
       } else if (polls > 256 && (polls & 255) == 0) {
-        const bool late = globaltimer_ns() - t0 > SPIN_TIMEOUT_NS;
+        const bool late = globaltimer_ns() - t0 > limit_ns;
         const bool failed = ld_relaxed_u64(&hdr[WS_STATUS]) != 0ull;
         if (__any_sync(0xffffffffu, late || failed)) return 0ull;
       }

@@ -70,6 +70,33 @@ __global__ void __launch_bounds__(32) k_selftest_copy(unsigned long long limit_n
   }
 }
 
+// One warp waits for what no other will say, as the encoder's warps do.  `what` 3: the
+// prefix of a chunk whose group the scanner never reaches; 4: the flag of a preceding
+// chunk (small inputs); 5: the start of a buffer in a batch.  result[0]: what the wait
+// returns, result[2]: nanoseconds.  `ws`: a zeroed workspace for 129 chunks.
+__global__ void __launch_bounds__(32) k_selftest_place_waits(int what, unsigned long long limit_ns, uint64_t* ws,
+                                                             long long* result)
+{
+  __shared__ ScanRing ring;
+  if (threadIdx.x == 0) {
+    ring.known = 0;
+    ring.gone = 0;
+  }
+  __syncwarp();
+  const ChunkScan scan(ws + WS_HDR_WORDS, 129, &ring);
+  const unsigned long long t0 = globaltimer_ns();
+  long long r = 0;
+  if (what == 3) r = scan.prefix(GROUP, 0, ws, limit_ns);
+  else if (what == 4) r = scan.prefix_flags(1, ws, limit_ns);
+  else r = static_cast<long long>(ChunkScan::await(ws + WS_HDR_WORDS, ws, limit_ns));
+  const unsigned long long t1 = globaltimer_ns();
+  if (threadIdx.x == 0) {
+    result[0] = r;
+    result[1] = 0;
+    result[2] = static_cast<long long>(t1 - t0);
+  }
+}
+
 // Two warps as a decode team: the wait of warp `what` (0 or 1) gives up, the other's
 // ends well.  result[0]: the status that the team leaves in `hdr`; result[1]: the
 // position; result[2]: nanoseconds
@@ -410,23 +437,25 @@ extern "C" int sleek_selftest_bounded_waits(long long limit_ns, long long* h_res
 
 extern "C" int sleek_selftest_wait(int what, long long limit_ns, long long* h_result)
 {
-  if (!h_result || what < 0 || what > 2 || limit_ns <= 0 || limit_ns > 1000000000ll) return SLEEK_ERR_INVALID_ARG;
+  if (!h_result || what < 0 || what > 5 || limit_ns <= 0 || limit_ns > 1000000000ll) return SLEEK_ERR_INVALID_ARG;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
     cudaGetLastError();
     return SLEEK_ERR_NO_DEVICE;
   }
-  uint64_t* d = nullptr;  // a zeroed workspace header
+  const size_t words = static_cast<size_t>(sleek::WS_HDR_WORDS + sleek::scan_words(129));
+  uint64_t* d = nullptr;  // a zeroed workspace
   long long* d_res = nullptr;
   int rc = SLEEK_OK;
-  if (cudaMalloc(&d, sleek::WS_HDR_WORDS * sizeof(uint64_t)) != cudaSuccess ||
+  if (cudaMalloc(&d, words * sizeof(uint64_t)) != cudaSuccess ||
       cudaMalloc(&d_res, 3 * sizeof(long long)) != cudaSuccess ||
-      cudaMemset(d, 0, sleek::WS_HDR_WORDS * sizeof(uint64_t)) != cudaSuccess) {
+      cudaMemset(d, 0, words * sizeof(uint64_t)) != cudaSuccess) {
     rc = SLEEK_ERR_CUDA;
   } else {
     const unsigned long long limit = static_cast<unsigned long long>(limit_ns);
     if (what < 2) sleek::k_selftest_team<<<1, 64>>>(what, limit, d, d_res);
-    else sleek::k_selftest_copy<<<1, 32>>>(limit, d_res);
+    else if (what == 2) sleek::k_selftest_copy<<<1, 32>>>(limit, d_res);
+    else sleek::k_selftest_place_waits<<<1, 32>>>(what, limit, d, d_res);
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
         cudaMemcpy(h_result, d_res, 3 * sizeof(long long), cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = SLEEK_ERR_CUDA;

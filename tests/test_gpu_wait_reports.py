@@ -28,3 +28,10 @@ def test_a_warp_waits_once_more_for_its_copy_before_it_leaves(cuda):
     landed, _, ns = run(2)
     assert landed == 0
     assert ns >= 2 * LIMIT
+
+
+@pytest.mark.parametrize("what, gives_up_with", [(3, -1), (4, -1), (5, 0)])
+def test_waits_for_a_chunks_place_give_up(cuda, what, gives_up_with):
+    got, _, ns = run(what)
+    assert got == gives_up_with
+    assert LIMIT <= ns < LIMIT + 2_000_000_000
