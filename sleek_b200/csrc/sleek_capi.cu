@@ -80,7 +80,7 @@ int persistent_grid(int dev, int width, bool lossy, bool enc, long long bytes, i
     d.sms = sms > 0 ? sms : 1;
   }
   Choice c = bytes < 0 ? Choice{} : d.choice[width == 8][lossy][enc][size_bucket(bytes)];
-  if (c.shape == 0 && c.ctas == 0 && bytes >= 0) c.shape = sleek::default_shape(enc, (bytes + CS - 1) / CS, d.sms);
+  if (c.shape == 0 && c.ctas == 0 && bytes >= 0) c.shape = sleek::default_shape(enc, sleek::chunks_of(bytes), d.sms);
   int& b = d.bps[width == 8][lossy][enc][c.shape];
   if (b == 0) {
     const int n = sleek::blocks_per_sm(width, lossy, enc, c.shape);
@@ -210,7 +210,7 @@ int do_decompress(int width, bool lossy, sleek::QParams q, const unsigned char* 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int shape = 0;
   int grid = persistent_grid(dev, width, lossy, false, out_cap >= 0 ? out_cap : in_len, &shape);
-  if (out_cap >= 0 && grid > (out_cap + CS - 1) / CS) grid = out_cap > 0 ? static_cast<int>((out_cap + CS - 1) / CS) : 1;
+  if (out_cap >= 0 && grid > sleek::chunks_of(out_cap)) grid = out_cap > 0 ? static_cast<int>(sleek::chunks_of(out_cap)) : 1;
   uint64_t* w = nullptr;
   long long cap = 0;
   rc = prepare_workspace(st, ws, wsb, grid, &w, &cap);

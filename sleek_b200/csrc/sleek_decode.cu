@@ -310,13 +310,13 @@ __global__ void __launch_bounds__(NTEAM * TW * 32, MINB) k_decode(const DecArgs 
   // sizes are added up while the header is still on its way, instead of one
   // dependent round trip after it.  Used only if the header agrees; the reads stay
   // inside the stated stream length.
-  const long long g_chunks = a.out_cap > 0 ? (a.out_cap + CS - 1) / CS : -1;
+  const long long g_chunks = a.out_cap > 0 ? chunks_of(a.out_cap) : -1;
   const bool spec = g_chunks > 0 && a.in_len >= 8 + 2 * g_chunks;
   const long long insize = *reinterpret_cast<const long long*>(a.in);
   if (spec) sum_groups(0, min(g_chunks, static_cast<long long>(DEC_WINDOW)));
 
   // header checks (every CTA reads the 8-byte header)
-  const long long chunks_in = insize > 0 ? (insize + CS - 1) / CS : 0;
+  const long long chunks_in = insize > 0 ? chunks_of(insize) : 0;
   bool hdr_ok = insize >= 0 && (insize % static_cast<long long>(sizeof(T))) == 0;
   if (a.in_len >= 0 && 8 + 2 * chunks_in > a.in_len) hdr_ok = false;
   const bool cap_ok = a.out_cap < 0 || insize <= a.out_cap;

@@ -9,6 +9,10 @@ struct sleek_stream_info;
 
 namespace sleek {
 
+// chunks of `bytes` >= 0 bytes, for any such count: a stream's header and a caller's
+// capacity may say anything up to 2^63 - 1
+constexpr long long chunks_of(long long bytes) { return bytes / 16384 + (bytes % 16384 != 0); }
+
 // lossy quantizer parameters, as sleek_error_bound derives them
 // (include/sleek_lossy_gpu.h:47-71 of the reference)
 struct QParams {

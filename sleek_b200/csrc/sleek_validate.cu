@@ -64,7 +64,7 @@ int sleek::validate_stream(const unsigned char* s, long long len, int elem_bytes
     fail(info, SLEEK_STREAM_BAD_SIZE, -1);
     return SLEEK_ERR_CORRUPT_STREAM;
   }
-  const long long chunks = (insize + CS - 1) / CS;
+  const long long chunks = sleek::chunks_of(insize);
   info->chunks = chunks;
   if (chunks > (len - 8) / 2) {
     fail(info, SLEEK_STREAM_SHORT_TABLE, -1);
