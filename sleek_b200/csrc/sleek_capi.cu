@@ -68,9 +68,12 @@ int current_device(int* dev)
   return SLEEK_OK;
 }
 
-// Persistent grid and launch shape of a single-buffer call of `bytes` bytes
-// (bytes < 0: unknown, the default shape).
-int persistent_grid(int dev, int width, bool lossy, bool enc, long long bytes, int* shape)
+// Persistent grid and launch shape of a single-buffer call.  `bytes` picks the size
+// bucket of the choices made with sleek_set_launch_shape, `chunks` the form for small
+// inputs where none was made; -1: unknown (no choice, no such form).  They differ where a
+// decode states no capacity: a stream's length says little about its chunks (2 MB may
+// hold 200 MB of zeros).
+int persistent_grid(int dev, int width, bool lossy, bool enc, long long bytes, long long chunks, int* shape)
 {
   std::lock_guard<std::mutex> lk(g_mu);
   DeviceInfo& d = g_dev[dev];
@@ -80,7 +83,7 @@ int persistent_grid(int dev, int width, bool lossy, bool enc, long long bytes, i
     d.sms = sms > 0 ? sms : 1;
   }
   Choice c = bytes < 0 ? Choice{} : d.choice[width == 8][lossy][enc][size_bucket(bytes)];
-  if (c.shape == 0 && c.ctas == 0 && bytes >= 0) c.shape = sleek::default_shape(enc, sleek::chunks_of(bytes), d.sms);
+  if (c.shape == 0 && c.ctas == 0 && chunks >= 0) c.shape = sleek::default_shape(enc, chunks, d.sms);
   int& b = d.bps[width == 8][lossy][enc][c.shape];
   if (b == 0) {
     const int n = sleek::blocks_per_sm(width, lossy, enc, c.shape);
@@ -187,7 +190,7 @@ int do_compress(int width, bool lossy, sleek::QParams q, const void* in, long lo
   a.flag_cap = cap;
   a.q = q;
   int shape = 0;
-  long long grid = persistent_grid(dev, width, lossy, true, insize, &shape);
+  long long grid = persistent_grid(dev, width, lossy, true, insize, chunks, &shape);
   if (grid > chunks) grid = chunks > 0 ? chunks : 1;
   if (sleek::launch_encode(width, lossy, shape, a, static_cast<int>(grid), st) != cudaSuccess) {
     cudaGetLastError();
@@ -209,8 +212,9 @@ int do_decompress(int width, bool lossy, sleek::QParams q, const unsigned char* 
   if (rc) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int shape = 0;
-  int grid = persistent_grid(dev, width, lossy, false, out_cap >= 0 ? out_cap : in_len, &shape);
-  if (out_cap >= 0 && grid > sleek::chunks_of(out_cap)) grid = out_cap > 0 ? static_cast<int>(sleek::chunks_of(out_cap)) : 1;
+  const long long chunks = out_cap >= 0 ? sleek::chunks_of(out_cap) : -1;
+  int grid = persistent_grid(dev, width, lossy, false, out_cap >= 0 ? out_cap : in_len, chunks, &shape);
+  if (chunks >= 0 && grid > chunks) grid = chunks > 0 ? static_cast<int>(chunks) : 1;
   uint64_t* w = nullptr;
   long long cap = 0;
   rc = prepare_workspace(st, ws, wsb, grid, &w, &cap);
@@ -371,7 +375,7 @@ int sleek_thread_blocks(void)
   int dev = 0;
   if (current_device(&dev)) return 0;
   int shape = 0;
-  return persistent_grid(dev, 4, false, true, -1, &shape);
+  return persistent_grid(dev, 4, false, true, -1, -1, &shape);
 }
 
 size_t sleek_compress_workspace_size(long long insize) { return insize < 0 ? 0 : enc_ws_bytes(insize); }

@@ -42,3 +42,53 @@ def test_headers_beyond_the_stream_are_corrupt(cuda, insize):
         y, size = _decode(s, np.float64, 512, cap, len(s))
         assert size == -_capi.SLEEK_ERR_CORRUPT_STREAM
         assert np.all(y == 7.0)
+
+
+class _KernelNode(C.Structure):  # CUDA_KERNEL_NODE_PARAMS of the driver API
+    _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("smem", C.c_uint),
+                ("params", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+
+def _launched(call):
+    """(CTAs, threads per CTA) of the one kernel that `call` launches."""
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(g):
+        call()
+    cu = C.CDLL("libcuda.so.1")
+    graph = C.c_void_p(g.raw_cuda_graph())
+    n = C.c_size_t(0)
+    assert cu.cuGraphGetNodes(graph, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert cu.cuGraphGetNodes(graph, nodes, C.byref(n)) == 0
+    found = []
+    for node in nodes:
+        kind = C.c_int(-1)
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        if kind.value == 0:  # a kernel
+            p = _KernelNode()
+            assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) == 0
+            found.append((p.grid[0], p.block[0]))
+    assert len(found) == 1, found
+    return found[0]
+
+
+def test_small_form_goes_by_the_output_not_by_the_stream(cuda):
+    # 100 MB of zeros in 0.2 MB of stream: more chunks than SMs, a stream of a few chunks' length
+    n = 6400 * 4096
+    s = O.encode(np.zeros(n, np.float32))
+    t = torch.frombuffer(bytearray(s), dtype=torch.uint8).cuda()
+    out = torch.full((n,), 7.0, device="cuda")
+    size = torch.zeros(1, dtype=torch.int64, device="cuda")
+    L = _capi.lib()
+    ws = torch.empty(L.sleek_decompress_workspace_size(), dtype=torch.uint8, device="cuda")
+
+    def call(cap):
+        _capi.check(L.sleek_decompress_f32(t.data_ptr(), t.numel(), out.data_ptr(), cap, size.data_ptr(), ws.data_ptr(),
+                                           ws.numel(), torch.cuda.current_stream().cuda_stream))
+
+    known = _launched(lambda: call(n * 4))
+    assert _launched(lambda: call(-1)) == known
+    small = _launched(lambda: call(40 * 16384))  # (captured only: the stream does not fit)
+    assert small[1] != known[1]
+    call(-1)
+    assert int(size.item()) == n * 4 and not out.any()
