@@ -15,7 +15,8 @@ threads and a grid from ``sleek_thread_blocks``, include/sleek_common_gpu.h:54-5
 
 Candidates are timed with CUDA events on the caller's data (outputs are identical
 for every candidate), and the winner is cached per device name and key in a JSON
-file.
+file.  A shape is cached under a key that holds the library's whole table of shapes:
+its number means nothing to a library whose table is another.
 """
 from __future__ import annotations
 
@@ -104,6 +105,12 @@ def single_candidates(decompress: bool) -> List[tuple]:
     return out
 
 
+def single_key(decompress: bool, elem_bytes: int, lossy: bool, bucket: int) -> str:
+    """The cache key of a single-buffer choice."""
+    table = ",".join(f"{s['threads']}.{s['warps']}.{s['stages']}.{s['ctas_per_sm']}" for s in shapes(decompress))
+    return f"single|{'dec' if decompress else 'enc'}|{elem_bytes}|{int(lossy)}|2^{bucket}|{table}"
+
+
 def size_log2(nbytes: int) -> int:
     return max(0, int(nbytes).bit_length() - 1)
 
@@ -144,8 +151,7 @@ def tune_single(x: torch.Tensor, eb: Optional[float], decompress: bool = False, 
                 rc = fc(*pre, x.data_ptr(), x.numel(), buf.data_ptr(), size.data_ptr(), None, 0, sh)
             _capi.check(rc)
 
-    key = f"single|{'dec' if decompress else 'enc'}|{w}|{lossy}|2^{bucket}"
-    r = tune(key, run, single_candidates(decompress), use_cache=use_cache)
+    r = tune(single_key(decompress, w, lossy, bucket), run, single_candidates(decompress), use_cache=use_cache)
     apply(r["best"])
     r.update({"bucket_log2": bucket, "shape": shapes(decompress)[r["best"][0]]})
     return r
