@@ -34,11 +34,14 @@ class ErrorBoundInfo(NamedTuple):
     dtype: np.dtype
 
     def c_struct(self):
-        return _c_struct(self.eb_e, self.thr_e, self.offs_e, np.dtype(self.dtype).itemsize)
+        if self.dtype == np.float32:
+            return _capi.EbInfoF32(self.eb_e, self.thr_e, self.offs_e)
+        return _capi.EbInfoF64(self.eb_e, self.thr_e, self.offs_e)
 
 
 @lru_cache(maxsize=256)
-def _c_struct(eb_e, thr_e, offs_e, itemsize):
+def _eb_struct(eb_e, thr_e, offs_e, itemsize):
+    """A bound's c_struct, made once; for the calls below alone, which pass it by value."""
     return (_capi.EbInfoF32 if itemsize == 4 else _capi.EbInfoF64)(eb_e, thr_e, offs_e)
 
 
@@ -153,8 +156,8 @@ def sleek_compress_gpu(blocks: int, *args, stream=None, workspace=None, check: b
     else:
         if eb_info.dtype != dt:
             raise TypeError("eb_info dtype does not match the input dtype")
-        rc = _entry("compress", True, w)(eb_info.c_struct(), d_input.data_ptr(), n, d_encoded.data_ptr(),
-                                         d_encsize.data_ptr(), wp, wb, st)
+        eb = _eb_struct(eb_info.eb_e, eb_info.thr_e, eb_info.offs_e, w)
+        rc = _entry("compress", True, w)(eb, d_input.data_ptr(), n, d_encoded.data_ptr(), d_encsize.data_ptr(), wp, wb, st)
     if rc:
         _capi.check(rc, "sleek_compress_gpu")
     if check:
@@ -190,8 +193,9 @@ def sleek_decompress_gpu(blocks: int, *args, stream=None, workspace=None, check:
     else:
         if eb_info.dtype != dt:
             raise TypeError("eb_info dtype does not match the output dtype")
-        rc = _entry("decompress", True, w)(eb_info.c_struct(), d_encoded.data_ptr(), int(encoded_bytes),
-                                           d_decoded.data_ptr(), cap, d_decsize.data_ptr(), wp, wb, st)
+        eb = _eb_struct(eb_info.eb_e, eb_info.thr_e, eb_info.offs_e, w)
+        rc = _entry("decompress", True, w)(eb, d_encoded.data_ptr(), int(encoded_bytes), d_decoded.data_ptr(), cap,
+                                           d_decsize.data_ptr(), wp, wb, st)
     if rc:
         _capi.check(rc, "sleek_decompress_gpu")
     if check:
