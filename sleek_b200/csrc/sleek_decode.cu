@@ -31,15 +31,13 @@ constexpr int DEC_G = 4;  // subchunks whose loads and shifts overlap
 // This lane's 16 bytes of output values.
 __device__ __forceinline__ void store16(uint8_t* o, const uint4 v) { *reinterpret_cast<uint4*>(o) = v; }
 
-// The same where the output is not 16-byte aligned or the chunk ends before them:
-// 32-bit words, `have` bytes of them (a multiple of the element size).
-__device__ __forceinline__ void store_words(uint8_t* o, const uint4 v, int have)
+// The first `have` of them (4, 8 or 12), where the chunk ends.
+__device__ __forceinline__ void store_part(uint8_t* o, const uint4 v, int have)
 {
   uint32_t* const p = reinterpret_cast<uint32_t*>(o);
   if (have >= 4) p[0] = v.x;
   if (have >= 8) p[1] = v.y;
   if (have >= 12) p[2] = v.z;
-  if (have >= 16) p[3] = v.w;
 }
 
 // Values of the lane's codes.  W: the codes' widths are below 24 bits (32-bit values)
@@ -108,6 +106,19 @@ __device__ __forceinline__ uint4 codes_wide(const uint32_t* w, int bit, int ln, 
     return make_uint4(x0, x1 & m, __funnelshift_rc(x1, x2, k), __funnelshift_rc(x2, x3, k) & m);
   }
 }
+// one code at bit `at`, of any width
+template <typename T>
+__device__ __forceinline__ T code_at(const uint32_t* w, int at, int ln)
+{
+  const uint32_t* const p = w + (at >> 5);
+  const uint32_t lo = __funnelshift_r(p[0], p[1], at) & (pow2_or_0(ln) - 1u);
+  if constexpr (sizeof(T) == 4) {
+    return lo;
+  } else {
+    const uint32_t hi = ln > 32 ? __funnelshift_r(p[1], p[2], at) & (pow2_or_0(ln - 32) - 1u) : 0u;
+    return (static_cast<uint64_t>(hi) << 32) | lo;
+  }
+}
 // 16 raw bytes at any bit offset
 __device__ __forceinline__ uint4 codes_full(const uint32_t* w, int bit, int lane)
 {
@@ -116,6 +127,107 @@ __device__ __forceinline__ uint4 codes_full(const uint32_t* w, int bit, int lane
   const uint32_t w0 = p[0], w1 = p[1], w2 = p[2], w3 = p[3], w4 = p[4];
   return make_uint4(__funnelshift_r(w0, w1, at), __funnelshift_r(w1, w2, at), __funnelshift_r(w2, w3, at),
                     __funnelshift_r(w3, w4, at));
+}
+
+// A chunk whose output is not 16-byte aligned, or that ends early (a stream's last), with
+// the chunk already checked (`ln`: width of subchunk `lane`).  Each lane takes the values
+// of 16 aligned bytes of output, which begin `mis` bytes before those of an aligned
+// output; the values before a subchunk's first and after its last such granule follow one
+// by one, a lane each, for the whole chunk.  (302 MB f64 at eb 1e-4 into a view that begins
+// at element 1: 72 us, aligned 64; 26 MB f32 at eb 1e-3 13.7 and 12.6, 67 MB f32 lossless
+// 29.7 and 26.6, raw chunks 27.7 and 27.4.  With words at the lanes' own 16 bytes, which
+// fill a quarter of each sector per store, 89, 16.2, 29.8 and 30.3; with words moved between
+// the lanes by shuffles 99, 16.9, 37 and 27.9.)
+template <typename T, bool LOSSY, int TW>
+__device__ __forceinline__ void unpack_unaligned(const uint32_t* w, int sft, int ln, int osize, uint8_t* o, const QParams& q,
+                                              int cw, int lane)
+{
+  using V = VT<T>;
+  constexpr int B = static_cast<int>(sizeof(T));
+  constexpr int P = 16 / B;  // values per lane
+  constexpr int NARROW = B == 4 ? 16 : 32;
+  const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(o) & 15u);
+  const int m = mis / B;
+  const bool mine = lane > 0 || mis == 0;  // (else lane 0's first values are the subchunk's before)
+  const int last = mine ? osize - 16 - lane * 16 + mis : -1;  // the last subchunk's first byte that has all 16
+  const unsigned narrow = __ballot_sync(0xffffffffu, ln < NARROW);
+  const unsigned wide = __ballot_sync(0xffffffffu, ln >= NARROW);
+#pragma unroll 1
+  for (int g = cw; g < SC / DEC_G; g += TW) {
+    const int i0 = g * DEC_G;
+    const uint32_t lw = __reduce_or_sync(0xffffffffu, (lane / DEC_G) == g ? static_cast<uint32_t>(ln) << (8 * (lane % DEC_G)) : 0u);
+    int l[DEC_G], b[DEC_G];
+    int bit = 8 * sft + 256 + V::VPS * __reduce_add_sync(0xffffffffu, lane < i0 ? ln : 0);
+#pragma unroll
+    for (int u = 0; u < DEC_G; ++u) {
+      l[u] = static_cast<int>((lw >> (8 * u)) & 0xffu);
+      b[u] = bit;
+      bit += V::VPS * l[u];
+    }
+    constexpr unsigned ALL = (1u << DEC_G) - 1u;
+    const unsigned nm = (narrow >> i0) & ALL, wm = (wide >> i0) & ALL;
+    uint4 e[DEC_G];
+    if (nm == ALL) {
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) e[u] = codes_narrow<B>(w, b[u] - m * l[u], l[u], lane);
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) e[u] = decode_codes<T, LOSSY, true>(e[u], q);
+    } else if (wm == ALL) {
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) e[u] = codes_wide<B>(w, b[u] - m * l[u], l[u], lane);
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) e[u] = decode_codes<T, LOSSY, false>(e[u], q);
+    } else {
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) {
+        if ((nm >> u) & 1u) e[u] = codes_narrow<B>(w, b[u] - m * l[u], l[u], lane);
+        else e[u] = codes_wide<B>(w, b[u] - m * l[u], l[u], lane);
+      }
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) e[u] = decode_codes<T, LOSSY, false>(e[u], q);
+    }
+#pragma unroll
+    for (int u = 0; u < DEC_G; ++u)
+      if ((i0 + u) * 512 <= last) store16(o + (i0 + u) * 512 + lane * 16 - mis, e[u]);
+    if (osize < CS) {
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) {
+        const int at = (i0 + u) * 512 + lane * 16 - mis;
+        if (mine && at < osize && at + 16 > osize) store_part(o + at, e[u], osize - at);
+      }
+    }
+  }
+  if (mis != 0) {
+    int incl = ln;  // widths up to subchunk `lane`
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += x;
+    }
+    const int bit = 8 * sft + 256 + V::VPS * (incl - ln);
+    for (int j0 = cw * 32; j0 < SC * P; j0 += TW * 32) {
+      const int i = (j0 + lane) / P, t = (j0 + lane) % P;
+      const int k = t < P - m ? t : V::VPS - P + t;
+      const int l = __shfl_sync(0xffffffffu, ln, i);
+      const int at = __shfl_sync(0xffffffffu, bit, i) + k * l;
+      if (i * 512 + k * B < osize) *reinterpret_cast<T*>(o + i * 512 + k * B) = decode_value<LOSSY>(code_at<T>(w, at, l), q);
+    }
+  }
+}
+
+// A raw chunk to any output: the output's whole granules, then the words around them.
+template <int TW>
+__device__ __forceinline__ void copy_raw(const uint32_t* w, int sft, int osize, uint8_t* o, int cw, int lane)
+{
+  const int mis = static_cast<int>(reinterpret_cast<uintptr_t>(o) & 15u);
+  const int b = (16 - mis) & 15;  // bytes before the first granule (the chunk may end earlier)
+  const int e = max(b, ((mis + osize) & ~15) - mis);
+  for (int at = b + (cw * 32 + lane) * 16; at < e; at += TW * 512) store16(o + at, codes_full(w, 8 * (sft + at), 0));
+  if (cw == 0) {
+    const int at = lane < 4 ? 4 * lane : e + 4 * (lane - 4);
+    if (lane < 4 ? at < min(b, osize) : at < osize && lane < 8)
+      *reinterpret_cast<uint32_t*>(o + at) = code_at<uint32_t>(w, 8 * (sft + at), 32);
+  }
 }
 
 // Decodes one staged chunk (payload at byte `sft` of `stg`, `cs` bytes, `osize` bytes
@@ -135,14 +247,12 @@ __device__ __forceinline__ bool decode_chunk(const uint8_t* stg, int sft, int cs
   constexpr int B = static_cast<int>(sizeof(T));
   const uint32_t* const w = reinterpret_cast<const uint32_t*>(stg);
   const bool whole = osize == CS && (reinterpret_cast<uintptr_t>(o) & 15u) == 0u;
-  o += lane * 16;
-  const int left = osize - lane * 16;  // bytes from this lane's place in subchunk 0
   if (cs == osize) {
-    for (int i = cw; i * 512 < osize; i += TW) {
-      const uint4 v = codes_full(w, 8 * sft + i * 4096, lane);
-      if (whole) store16(o + i * 512, v);
-      else store_words(o + i * 512, v, left - i * 512);
+    if (!whole) {
+      copy_raw<TW>(w, sft, osize, o, cw, lane);
+      return true;
     }
+    for (int i = cw; i < SC; i += TW) store16(o + i * 512 + lane * 16, codes_full(w, 8 * sft + i * 4096, lane));
     return true;
   }
   const int ln = stg[sft + lane];
@@ -150,64 +260,62 @@ __device__ __forceinline__ bool decode_chunk(const uint8_t* stg, int sft, int cs
   bool ok = !__any_sync(0xffffffffu, ln > V::TB) && 34 + tot / 8 == cs;
   if (ok) ok = static_cast<int16_t>(stg[sft + cs - 2] | (stg[sft + cs - 1] << 8)) == osize;
   if (!ok) return false;
+  if (!whole) {
+    unpack_unaligned<T, LOSSY, TW>(w, sft, ln, osize, o, q, cw, lane);
+    return true;
+  }
+  o += lane * 16;
   // widths of the narrow form, of the wide one, and (32-bit values) without escapes
   constexpr int NARROW = B == 4 ? 16 : 32;
   const unsigned narrow = __ballot_sync(0xffffffffu, ln < NARROW);
   const unsigned wide = __ballot_sync(0xffffffffu, ln >= NARROW);
   const unsigned plain = B == 4 && LOSSY ? __ballot_sync(0xffffffffu, ln < 24) : narrow;
-  auto unpack = [&](auto full) {
-    auto put = [&](int i, const uint4 v) {
-      if (decltype(full)::value) store16(o + i * 512, v);
-      else store_words(o + i * 512, v, left - i * 512);
-    };
+  auto put = [&](int i, const uint4 v) { store16(o + i * 512, v); };
 #pragma unroll 1
-    for (int g = cw; g < SC / DEC_G; g += TW) {
-      const int i0 = g * DEC_G;
-      // the group's widths as one warp-uniform word, so that what follows from them
-      // is computed once per warp, beside the lanes' own arithmetic
-      const uint32_t lw = __reduce_or_sync(0xffffffffu, (lane / DEC_G) == g ? static_cast<uint32_t>(ln) << (8 * (lane % DEC_G)) : 0u);
-      int l[DEC_G], b[DEC_G];
-      int bit = 8 * sft + 256 + V::VPS * __reduce_add_sync(0xffffffffu, lane < i0 ? ln : 0);
+  for (int g = cw; g < SC / DEC_G; g += TW) {
+    const int i0 = g * DEC_G;
+    // the group's widths as one warp-uniform word, so that what follows from them
+    // is computed once per warp, beside the lanes' own arithmetic
+    const uint32_t lw = __reduce_or_sync(0xffffffffu, (lane / DEC_G) == g ? static_cast<uint32_t>(ln) << (8 * (lane % DEC_G)) : 0u);
+    int l[DEC_G], b[DEC_G];
+    int bit = 8 * sft + 256 + V::VPS * __reduce_add_sync(0xffffffffu, lane < i0 ? ln : 0);
 #pragma unroll
-      for (int u = 0; u < DEC_G; ++u) {
-        l[u] = static_cast<int>((lw >> (8 * u)) & 0xffu);
-        b[u] = bit;
-        bit += V::VPS * l[u];
-      }
-      constexpr unsigned ALL = (1u << DEC_G) - 1u;
-      const unsigned nm = (narrow >> i0) & ALL, wm = (wide >> i0) & ALL, pm = (plain >> i0) & ALL;
-      uint4 e[DEC_G];
-      if (nm == ALL) {
+    for (int u = 0; u < DEC_G; ++u) {
+      l[u] = static_cast<int>((lw >> (8 * u)) & 0xffu);
+      b[u] = bit;
+      bit += V::VPS * l[u];
+    }
+    constexpr unsigned ALL = (1u << DEC_G) - 1u;
+    const unsigned nm = (narrow >> i0) & ALL, wm = (wide >> i0) & ALL, pm = (plain >> i0) & ALL;
+    uint4 e[DEC_G];
+    if (nm == ALL) {
 #pragma unroll
-        for (int u = 0; u < DEC_G; ++u) e[u] = codes_narrow<B>(w, b[u], l[u], lane);
+      for (int u = 0; u < DEC_G; ++u) e[u] = codes_narrow<B>(w, b[u], l[u], lane);
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) put(i0 + u, decode_codes<T, LOSSY, true>(e[u], q));
+    } else if (wm == ALL) {
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) e[u] = codes_wide<B>(w, b[u], l[u], lane);
+      if (B == 4 && LOSSY && pm == ALL) {
 #pragma unroll
         for (int u = 0; u < DEC_G; ++u) put(i0 + u, decode_codes<T, LOSSY, true>(e[u], q));
-      } else if (wm == ALL) {
-#pragma unroll
-        for (int u = 0; u < DEC_G; ++u) e[u] = codes_wide<B>(w, b[u], l[u], lane);
-        if (B == 4 && LOSSY && pm == ALL) {
-#pragma unroll
-          for (int u = 0; u < DEC_G; ++u) put(i0 + u, decode_codes<T, LOSSY, true>(e[u], q));
-        } else {
-#pragma unroll
-          for (int u = 0; u < DEC_G; ++u) put(i0 + u, decode_codes<T, LOSSY, false>(e[u], q));
-        }
       } else {
 #pragma unroll
-        for (int u = 0; u < DEC_G; ++u) {
-          if (l[u] < NARROW) e[u] = codes_narrow<B>(w, b[u], l[u], lane);
-          else e[u] = codes_wide<B>(w, b[u], l[u], lane);
-        }
+        for (int u = 0; u < DEC_G; ++u) put(i0 + u, decode_codes<T, LOSSY, false>(e[u], q));
+      }
+    } else {
 #pragma unroll
-        for (int u = 0; u < DEC_G; ++u) {
-          if (!LOSSY || ((pm >> u) & 1u)) put(i0 + u, decode_codes<T, LOSSY, true>(e[u], q));
-          else put(i0 + u, decode_codes<T, LOSSY, false>(e[u], q));
-        }
+      for (int u = 0; u < DEC_G; ++u) {
+        if (l[u] < NARROW) e[u] = codes_narrow<B>(w, b[u], l[u], lane);
+        else e[u] = codes_wide<B>(w, b[u], l[u], lane);
+      }
+#pragma unroll
+      for (int u = 0; u < DEC_G; ++u) {
+        if (!LOSSY || ((pm >> u) & 1u)) put(i0 + u, decode_codes<T, LOSSY, true>(e[u], q));
+        else put(i0 + u, decode_codes<T, LOSSY, false>(e[u], q));
       }
     }
-  };
-  if (whole) unpack(std::true_type{});
-  else unpack(std::false_type{});
+  }
   return true;
 }
 
