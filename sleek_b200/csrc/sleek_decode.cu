@@ -31,14 +31,6 @@ constexpr int DEC_G = 4;  // subchunks whose loads and shifts overlap
 // This lane's 16 bytes of output values.
 __device__ __forceinline__ void store16(uint8_t* o, const uint4 v) { *reinterpret_cast<uint4*>(o) = v; }
 
-// The first `have` of them (4, 8 or 12), where the chunk ends.
-__device__ __forceinline__ void store_part(uint8_t* o, const uint4 v, int have)
-{
-  uint32_t* const p = reinterpret_cast<uint32_t*>(o);
-  if (have >= 4) p[0] = v.x;
-  if (have >= 8) p[1] = v.y;
-  if (have >= 12) p[2] = v.z;
-}
 
 // Values of the lane's codes.  W: the codes' widths are below 24 bits (32-bit values)
 // or 32 bits (64-bit values), so that no code is an escape.
@@ -134,7 +126,7 @@ __device__ __forceinline__ uint4 codes_full(const uint32_t* w, int bit, int lane
 // of 16 aligned bytes of output, which begin `mis` bytes before those of an aligned
 // output; the values before a subchunk's first and after its last such granule follow one
 // by one, a lane each, for the whole chunk.  (302 MB f64 at eb 1e-4 into a view that begins
-// at element 1: 72 us, aligned 64; 26 MB f32 at eb 1e-3 13.7 and 12.6, 67 MB f32 lossless
+// at element 1: 74 us, aligned 64; 26 MB f32 at eb 1e-3 13.7 and 12.6, 67 MB f32 lossless
 // 29.7 and 26.6, raw chunks 27.7 and 27.4.  With words at the lanes' own 16 bytes, which
 // fill a quarter of each sector per store, 89, 16.2, 29.8 and 30.3; with words moved between
 // the lanes by shuffles 99, 16.9, 37 and 27.9.)
@@ -189,13 +181,15 @@ __device__ __forceinline__ void unpack_unaligned(const uint32_t* w, int sft, int
 #pragma unroll
     for (int u = 0; u < DEC_G; ++u)
       if ((i0 + u) * 512 <= last) store16(o + (i0 + u) * 512 + lane * 16 - mis, e[u]);
-    if (osize < CS) {
-#pragma unroll
-      for (int u = 0; u < DEC_G; ++u) {
-        const int at = (i0 + u) * 512 + lane * 16 - mis;
-        if (mine && at < osize && at + 16 > osize) store_part(o + at, e[u], osize - at);
-      }
-    }
+  }
+  auto one = [&](int at, int bit, int l) { *reinterpret_cast<T*>(o + at) = decode_value<LOSSY>(code_at<T>(w, bit, l), q); };
+  const int tail = (osize + mis) & 15;  // the chunk's bytes in the granule that it ends in
+  if (tail != 0 && cw == 0) {
+    const int at = osize - tail + lane * B;
+    const int i = (osize - B) / 512;  // (earlier subchunks' values follow below)
+    const int l = __shfl_sync(0xffffffffu, ln, i);
+    const int bit = 8 * sft + 256 + V::VPS * __reduce_add_sync(0xffffffffu, lane < i ? ln : 0);
+    if (at < osize && at >= i * 512) one(at, bit + (at - i * 512) / B * l, l);
   }
   if (mis != 0) {
     int incl = ln;  // widths up to subchunk `lane`
@@ -210,7 +204,7 @@ __device__ __forceinline__ void unpack_unaligned(const uint32_t* w, int sft, int
       const int k = t < P - m ? t : V::VPS - P + t;
       const int l = __shfl_sync(0xffffffffu, ln, i);
       const int at = __shfl_sync(0xffffffffu, bit, i) + k * l;
-      if (i * 512 + k * B < osize) *reinterpret_cast<T*>(o + i * 512 + k * B) = decode_value<LOSSY>(code_at<T>(w, at, l), q);
+      if (i * 512 + k * B < osize) one(i * 512 + k * B, at, l);
     }
   }
 }
@@ -875,9 +869,9 @@ ShapeInfo shape_info(bool enc, int shape)
 
 int shape_count(bool enc) { return enc ? encode_shape_count() : DEC_SHAPES; }
 
-// Decode with at most one chunk per SM: shape 2, whose eight warps share a chunk (f32
-// lossless, microseconds on the GPU against shape 0's: 200 KB 6.0 / 6.5, 1.6 MB 6.1 /
-// 6.4; with more chunks its larger CTAs cost more than they gain: 3 MB 7.6 / 6.1).
+// Decode with at most one chunk per SM: shape 2, whose eight warps share a chunk (f32 lossless,
+// microseconds on the GPU against shape 0's: 200 KB 6.0 / 6.5, 1.6 MB 6.1 / 6.4; with more
+// chunks its larger CTAs cost more than they gain: 3 MB 7.6 / 6.1).
 int default_shape(bool enc, long long chunks, int sms)
 {
   if (enc) return encode_default_shape(chunks, sms);

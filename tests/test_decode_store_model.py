@@ -1,8 +1,8 @@
 """CPU model of the decoder's stores into outputs that are not 16-byte aligned, and of a
 stream's partial last chunk (unpack_unaligned and copy_raw in
 sleek_b200/csrc/sleek_decode.cu): the kernel's index arithmetic, lane by lane, with the
-chunk's own byte positions as the values.  Every byte of the chunk is written once, with
-its own value, nothing outside the chunk is written, and 16-byte stores are aligned."""
+chunk's own byte positions as the values.  Every byte of the chunk is written, with its
+own value, nothing outside the chunk is written, and 16-byte stores are aligned."""
 import pytest
 
 CS, SC, G = 16384, 32, 4
@@ -21,10 +21,10 @@ class Out:
         assert at not in self.words
         self.words[at] = value
 
-    def part(self, at, v, have):
-        assert have in (4, 8, 12)
-        for k in range(have // 4):
-            self.word(at + 4 * k, v[k])
+    def value(self, at, width):
+        for h in range(0, width, 4):
+            assert self.words.get(at + h, at + h) == at + h  # (again with the same value, if at all)
+            self.words[at + h] = at + h
 
     def check(self, osize):
         assert sorted(self.words) == list(range(0, osize, 4))
@@ -52,8 +52,14 @@ def test_unpacked_chunks(width, mis):
                 if i * 512 <= last:
                     assert 0 <= first and first + P <= VPS
                     out.store16(at, v)
-                if mine and at < osize < at + 16:
-                    out.part(at, v, osize - at)
+        tail = (osize + mis) & 15
+        if tail:
+            i = (osize - width) // 512
+            for lane in range(32):
+                at = osize - tail + lane * width
+                if i * 512 <= at < osize:
+                    assert at < (i + 1) * 512
+                    out.value(at, width)
         if mis:
             for i0 in range(0, SC, G):
                 for lane in range(G * P):
@@ -61,8 +67,7 @@ def test_unpacked_chunks(width, mis):
                     k = t if t < P - m else VPS - P + t
                     at = (i0 + u) * 512 + k * width
                     if at < osize:
-                        for h in range(0, width, 4):
-                            out.word(at + h, at + h)
+                        out.value(at, width)
         out.check(osize)
 
 
