@@ -802,6 +802,11 @@ using DecShape0 = DecShape<6, 2, 1>;  // default
 using DecShape1 = DecShape<10, 1, 1>;
 using DecShape2 = DecShape<2, 8, 2>;
 constexpr int DEC_SHAPES = 3;
+// Index DEC_SHAPES, past the shapes that can be asked for: shape 2 for at most one chunk
+// per SM, with the registers of one CTA per SM.  With those of two, some of which are
+// spilled, one 4 KB chunk takes 5.03 us on the GPU instead of 4.86, but large inputs that
+// ask for shape 2 want two CTAs (302 MB f64 at eb 1e-4 87 us, 110 with one).
+using DecShapeSmall = DecShape<2, 8, 1>;
 
 template <typename T, bool LOSSY, class S>
 static cudaError_t launch_dec_k(const DecArgs& a, int grid, cudaStream_t st)
@@ -829,6 +834,7 @@ static cudaError_t launch_dec_kind(int shape, const DecArgs& a, int grid, cudaSt
   switch (shape) {
     case 1: return launch_dec_k<T, LOSSY, DecShape1>(a, grid, st);
     case 2: return launch_dec_k<T, LOSSY, DecShape2>(a, grid, st);
+    case DEC_SHAPES: return launch_dec_k<T, LOSSY, DecShapeSmall>(a, grid, st);
     default: return launch_dec_k<T, LOSSY, DecShape0>(a, grid, st);
   }
 }
@@ -839,6 +845,7 @@ static int dec_occupancy_kind(int shape)
   switch (shape) {
     case 1: return dec_occupancy<T, LOSSY, DecShape1>();
     case 2: return dec_occupancy<T, LOSSY, DecShape2>();
+    case DEC_SHAPES: return dec_occupancy<T, LOSSY, DecShapeSmall>();
     default: return dec_occupancy<T, LOSSY, DecShape0>();
   }
 }
@@ -869,13 +876,13 @@ ShapeInfo shape_info(bool enc, int shape)
 
 int shape_count(bool enc) { return enc ? encode_shape_count() : DEC_SHAPES; }
 
-// Decode with at most one chunk per SM: shape 2, whose eight warps share a chunk (f32 lossless,
+// Decode with at most one chunk per SM: eight warps share a chunk (f32 lossless,
 // microseconds on the GPU against shape 0's: 200 KB 6.0 / 6.5, 1.6 MB 6.1 / 6.4; with more
 // chunks its larger CTAs cost more than they gain: 3 MB 7.6 / 6.1).
 int default_shape(bool enc, long long chunks, int sms)
 {
   if (enc) return encode_default_shape(chunks, sms);
-  return chunks <= sms ? 2 : 0;
+  return chunks <= sms ? DEC_SHAPES : 0;
 }
 
 cudaError_t launch_decode_batch(const BatchDecArgs& a, int grid, cudaStream_t st)
