@@ -15,7 +15,8 @@
  *
  * Pointers: device inputs/outputs must be aligned to their element size (4 for
  * float, 8 for double); the stream buffer must be 8-byte aligned.  16-byte
- * aligned inputs take the TMA path; others are copied 4 bytes at a time.
+ * aligned inputs take the TMA path; others, and the last partial chunk, are copied 16, 8 or
+ * 4 bytes at a time.
  *
  * Workspace: pass NULL to use a workspace the library owns (one per device and
  * stream, grown on demand -- growth calls cudaMalloc, so size it up front with a

@@ -8,12 +8,12 @@
 // stores.  No CTA waits for another, and there is no CTA barrier per chunk.  Malformed
 // streams set an error status instead of trapping; every wait is bounded.
 //
-// What bounds it: HBM on large fields (302 MB f64 at eb 1e-4: 73.0 -> 63.6 us, 0.91 of
+// What bounds it: HBM on large fields (302 MB f64 at eb 1e-4: 73.2 -> 63.3 us, 0.91 of
 // the measured copy rate), else the waits at the start (header and table, the first
-// chunks' copies) and the ALU pipe (26 MB f32 at eb 1e-3: 18.2 -> 11.5 us; 67 MB f32
-// lossless: 29.7 -> 26.5 us; batch of 60 arrays: 60.7 -> 50.4 us).
-// A chunk costs 1,300 warp instructions (f64, eb 1e-4), 2,720 when eight warps shared
-// it and each lane took every 32nd value.
+// chunks' copies) and the ALU pipe (26 MB f32 at eb 1e-3: 17.9 -> 11.6 us; 67 MB f32
+// lossless: 29.9 -> 26.4 us; batch of 60 arrays: 61.4 -> 49.3 us).
+// A chunk costs 1,740 warp instructions (f64, eb 1e-4; all of the launch's), 2,720 when
+// eight warps shared it and each lane took every 32nd value.
 #include <type_traits>
 
 #include "sleek_device.cuh"
@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(PRE_NT) k_decode_prepass(const BatchDecArgs a)
 {
   __shared__ uint32_t wsum[PRE_NT / 32];
   __shared__ int wbad[PRE_NT / 32];
-  grid_release();
+  grid_release();  // at once: the decode kernel, which follows, is set up meanwhile (at the end instead: no change)
   grid_wait();
   const int j = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -701,7 +701,6 @@ __global__ void __launch_bounds__(DB_NT, 1) k_decode_batch(const BatchDecArgs a)
     if (leads) ticket = atomicAdd(reinterpret_cast<unsigned long long*>(&ws[WS_TICKET]), 1ull);
   };
   auto drawn = [&]() -> long long {
-    if constexpr (DB_TW == 1) return static_cast<long long>(__shfl_sync(0xffffffffu, ticket, 0));
     if (leads) s_ticket[turn][team] = ticket;
     team_failed<DB_TW>(team, false);
     const long long t = static_cast<long long>(s_ticket[turn][team]);

@@ -516,7 +516,7 @@ __device__ __forceinline__ uint64_t quant_fp(uint64_t val, const QParams& q)
 }
 
 // (A code of 0 needs no test: a, the product and the sign are 0.  Without the branch
-// 128 MB of escaped f32 values decode in 48 us instead of 68.)
+// 2^25 f32 values of random bits at eb 1e-3, nearly all escapes, decode in 48 us, not 68.)
 __device__ __forceinline__ uint32_t dequant_fp(uint32_t enc, const QParams& q)
 {
   const uint32_t a = (enc + 1u) >> 1;
@@ -840,8 +840,8 @@ struct ChunkScan {
 // to the arbitrary global byte address `dst`.  Whole aligned 16-byte granules
 // get one vector store each, funnel-shifted from two aligned shared loads; the
 // at most two granules shared with neighbouring chunks are written byte by
-// byte.  Called by NT threads with tid = 0 .. NT-1 (the encoder: its producer
-// warp, NT = 32).
+// byte.  Called by NT threads with tid = 0 .. NT-1: the warp of a raw chunk
+// (NT = 32), the team of a small input's chunk (NT = 256).
 // ----------------------------------------------------------------------------
 template <int WQ>
 __device__ __forceinline__ uint4 shifted_granule(const uint4 x, const uint4 y, int bb8)

@@ -18,7 +18,7 @@
 // published size and the store counts against the stages, so the pack comes before
 // the wait for the place, at the alignment the place is expected to have.
 // (302 MB f64 field: lossless 144 -> 111 us, eb 1e-4 130 -> 89 us; 26 MB f32 field,
-// eb 1e-3: 24.1 -> 12.9 us; 67 MB f32 signal, lossless: 44.6 -> 31.8 us.)
+// eb 1e-3: 24.0 -> 13.2 us; 67 MB f32 signal, lossless: 44.6 -> 31.8 us.)
 #include <type_traits>
 
 #include "sleek_device.cuh"

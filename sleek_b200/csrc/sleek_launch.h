@@ -1,5 +1,5 @@
 // sleek_launch.h -- host-side launch interface between the C ABI (sleek_capi.cu)
-// and the kernels (sleek_decode.cu).  Internal to the library.
+// and the kernels (sleek_encode.cu, sleek_decode.cu, sleek_reduce.cu).  Internal to the library.
 #pragma once
 
 #include <cstdint>

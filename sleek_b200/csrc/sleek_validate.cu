@@ -1,7 +1,7 @@
 // sleek_validate.cu -- host-side parser and checker of the stream format
 // (int64 original size | uint16 csize[chunks] | payloads, a compressed payload
 // being 32 x uint8 bit width | packed bits | int16 byte count).  The rules are the
-// ones the device decoders enforce (sleek_kernels.cu), checked in stream order so
+// ones the device decoders enforce (sleek_decode.cu), checked in stream order so
 // that the first malformed chunk is the one reported.
 #include <cstdint>
 #include <cstring>
