@@ -143,8 +143,9 @@ int sleek_decompress_lossy_f64(sleek_eb_info_f64 eb, const unsigned char* d_enco
 int sleek_compress_f32_static(const float* d_input, long long num_elements, unsigned char* d_encoded,
                               long long* d_encsize, void* stream);
 
-/* Tuning: CTAs per SM used by the single-buffer entry points of one kind on the current
- * device, for every input size (0 = as many as fit, the default).  Set by
+/* Tuning: CTAs per SM used at most by the single-buffer entry points of one kind on the
+ * current device, for every input size (0 = as many as fit, the default), in whatever shape
+ * they run (the forms for small inputs run where they keep within it).  Set by
  * sleek_b200.autotune; no counterpart in the reference, whose grid size comes from
  * sleek_thread_blocks and whose block size is the constant SLEEK_TPB
  * (include/sleek_common_gpu.h:54-56, 108-119). */
@@ -152,9 +153,9 @@ int sleek_set_ctas_per_sm(int decompress, int elem_bytes, int lossy, int ctas_pe
 
 /* Tuning: launch shapes.  The single-buffer kernels are built in a few shapes (threads per
  * CTA, warps that work on chunks, shared-memory chunk stages, and the CTAs per SM their
- * registers are budgeted for); shape 0 is the default -- with as many CTAs as fit it also
- * stands for the kernels' small-input forms, by the number of chunks -- and every shape
- * writes the same bytes.
+ * registers are budgeted for); shape 0 is the default -- unless it
+ * is selected with CTAs per SM here, it also stands for the kernels' small-input forms, by
+ * the number of chunks -- and every shape writes the same bytes.
  * sleek_launch_shape_info describes shape `shape` of the compress (decompress = 0) or
  * decompress kernels (any output pointer may be NULL) and returns SLEEK_ERR_INVALID_ARG
  * past the last one.  sleek_set_launch_shape selects the shape and the CTAs per SM (0 = as

@@ -30,7 +30,8 @@ constexpr int BUCKETS = 64;  // input sizes by their base-2 logarithm
 // what the single-buffer calls of one kind launch for one size bucket
 struct Choice {
   int shape = 0;  // launch shape (EncShape*, DecShape*)
-  int ctas = 0;   // CTAs per SM, 0 = as many as fit
+  int ctas = 0;   // CTAs per SM at most, 0 = as many as fit
+  bool fixed = false;  // a shape, or shape 0's CTAs, was asked for: no form for small inputs
 };
 
 struct DeviceInfo {
@@ -83,7 +84,7 @@ int persistent_grid(int dev, int width, bool lossy, bool enc, long long bytes, l
     d.sms = sms > 0 ? sms : 1;
   }
   Choice c = bytes < 0 ? Choice{} : d.choice[width == 8][lossy][enc][size_bucket(bytes)];
-  if (c.shape == 0 && c.ctas == 0 && chunks >= 0) c.shape = sleek::default_shape(enc, chunks, d.sms);
+  if (!c.fixed && chunks >= 0) c.shape = sleek::default_shape(enc, chunks, d.sms, c.ctas);
   int& b = d.bps[width == 8][lossy][enc][c.shape];
   if (b == 0) {
     const int n = sleek::blocks_per_sm(width, lossy, enc, c.shape);
@@ -484,7 +485,10 @@ int sleek_set_ctas_per_sm(int decompress, int elem_bytes, int lossy, int ctas_pe
   const int rc = current_device(&dev);
   if (rc) return rc;
   std::lock_guard<std::mutex> lk(g_mu);
-  for (Choice& c : g_dev[dev].choice[elem_bytes == 8][lossy != 0][decompress == 0]) c.ctas = ctas_per_sm;
+  for (Choice& c : g_dev[dev].choice[elem_bytes == 8][lossy != 0][decompress == 0]) {
+    c.ctas = ctas_per_sm;
+    c.fixed = c.shape != 0;
+  }
   return SLEEK_OK;
 }
 
@@ -510,7 +514,7 @@ int sleek_set_launch_shape(int decompress, int elem_bytes, int lossy, int size_l
   std::lock_guard<std::mutex> lk(g_mu);
   Choice* row = g_dev[dev].choice[elem_bytes == 8][lossy != 0][decompress == 0];
   for (int b = 0; b < BUCKETS; ++b)
-    if (size_log2 < 0 || b == size_log2) row[b] = Choice{shape, ctas_per_sm};
+    if (size_log2 < 0 || b == size_log2) row[b] = Choice{shape, ctas_per_sm, shape != 0 || ctas_per_sm != 0};
   return SLEEK_OK;
 }
 

@@ -878,9 +878,9 @@ int shape_count(bool enc) { return enc ? encode_shape_count() : DEC_SHAPES; }
 // Decode with at most one chunk per SM: eight warps share a chunk (f32 lossless,
 // microseconds on the GPU against shape 0's: 200 KB 6.0 / 6.5, 1.6 MB 6.1 / 6.4; with more
 // chunks its larger CTAs cost more than they gain: 3 MB 7.6 / 6.1).
-int default_shape(bool enc, long long chunks, int sms)
+int default_shape(bool enc, long long chunks, int sms, int ctas)
 {
-  if (enc) return encode_default_shape(chunks, sms);
+  if (enc) return encode_default_shape(chunks, sms, ctas);
   return chunks <= sms ? DEC_SHAPES : 0;
 }
 

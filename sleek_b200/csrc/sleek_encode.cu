@@ -959,9 +959,10 @@ int encode_shape_count() { return ENC_SHAPES; }
 
 // index ENC_SHAPES, past the shapes that can be asked for, is k_encode_team: its grid
 // has to be the number of chunks
-int encode_default_shape(long long chunks, int sms)
+int encode_default_shape(long long chunks, int sms, int ctas)
 {
-  return chunks <= static_cast<long long>(ENC_TEAM_CTAS) * sms ? ENC_SHAPES : 0;
+  const int most = ctas > 0 && ctas < ENC_TEAM_CTAS ? ctas : ENC_TEAM_CTAS;
+  return chunks <= static_cast<long long>(most) * sms ? ENC_SHAPES : 0;
 }
 
 ShapeInfo encode_shape_info(int shape)

@@ -84,13 +84,14 @@ struct ShapeInfo {
 };
 int shape_count(bool enc);
 // the shape that stands for shape 0 where no other was asked for, by the number of chunks
-int default_shape(bool enc, long long chunks, int sms);
+// and the CTAs per SM allowed (0: any number)
+int default_shape(bool enc, long long chunks, int sms, int ctas);
 ShapeInfo shape_info(bool enc, int shape);
 cudaError_t launch_encode(int width, bool lossy, int shape, const EncArgs& a, int grid, cudaStream_t st);
 cudaError_t launch_decode(int width, bool lossy, int shape, const DecArgs& a, int grid, cudaStream_t st);
 int blocks_per_sm(int width, bool lossy, bool enc, int shape);
 int encode_shape_count();
-int encode_default_shape(long long chunks, int sms);
+int encode_default_shape(long long chunks, int sms, int ctas);
 ShapeInfo encode_shape_info(int shape);
 int encode_blocks_per_sm(int width, bool lossy, int shape);
 cudaError_t launch_decode_batch(const BatchDecArgs& a, int grid, cudaStream_t st);
